@@ -18,6 +18,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "stretch.cuh"
 #include "svd.cuh"
 
 namespace slosh {
@@ -194,6 +195,23 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
     recompose<D>(sv.U, ns, sv.V, F);
 }
 
+// The models that take principal stretches, through the SVD of F: strains
+// outside the range of stretch.cuh (rare: kept out of line, so that its
+// registers are not the particle update's).
+template <int D>
+__device__ __noinline__ void model_update_svd(const Material &mat, uint32_t tag, float (&F)[D][D], float *st,
+                                              float (&tau)[D][D], unsigned *fp64) {
+    SvdD<D> sv;
+    sv.compute(F, fp64);
+    if (tag != SLOSH_MODEL_ELASTIC_LINEAR && mat.p[7] != 0.f) drucker_prager<D>(st, mat.p + 3, sv, F);
+    if (tag == SLOSH_MODEL_SAND_NEO_HOOKEAN) {
+        neo_hookean<D>(F, mat.p[9], mat.p[10], tau);
+    } else {
+        const float *el = tag == SLOSH_MODEL_ELASTIC_LINEAR ? mat.p : mat.p + 9;
+        fixed_corotated<D>(sv, el[0], el[1], tau);
+    }
+}
+
 // DefaultParticleModel::update (shaders/slosh/models/default.slang:51-92)
 // plus the Tait fluid.  `st` is the particle's plastic state (sand only).
 // `tag` is the material's model tag (a constant when the kernel is
@@ -202,31 +220,9 @@ template <int D>
 __device__ __forceinline__ void model_update(const Material &mat, uint32_t tag, float (&F)[D][D], float *st,
                                              float (&tau)[D][D], unsigned *fp64) {
     switch (tag) {
-        case SLOSH_MODEL_ELASTIC_LINEAR: {
-            SvdD<D> sv;
-            sv.compute(F, fp64);
-            fixed_corotated<D>(sv, mat.p[0], mat.p[1], tau);
-            break;
-        }
         case SLOSH_MODEL_ELASTIC_NEO_HOOKEAN:
             neo_hookean<D>(F, mat.p[0], mat.p[1], tau);
-            break;
-        case SLOSH_MODEL_SAND_LINEAR: {
-            SvdD<D> sv;
-            sv.compute(F, fp64);
-            if (mat.p[7] != 0.f) drucker_prager<D>(st, mat.p + 3, sv, F);
-            fixed_corotated<D>(sv, mat.p[9], mat.p[10], tau);
-            break;
-        }
-        case SLOSH_MODEL_SAND_NEO_HOOKEAN: {
-            if (mat.p[7] != 0.f) {
-                SvdD<D> sv;
-                sv.compute(F, fp64);
-                drucker_prager<D>(st, mat.p + 3, sv, F);
-            }
-            neo_hookean<D>(F, mat.p[9], mat.p[10], tau);
-            break;
-        }
+            return;
         case SLOSH_MODEL_FLUID_TAIT: {
             const float J = F[0][0];
             const float pressure = (mat.p[1] / mat.p[2]) * (powf(J, -mat.p[2]) - 1.f);
@@ -234,14 +230,55 @@ __device__ __forceinline__ void model_update(const Material &mat, uint32_t tag, 
             for (int i = 0; i < D; ++i)
 #pragma unroll
                 for (int k = 0; k < D; ++k) tau[i][k] = (i == k) ? -J * pressure : 0.f;
-            break;
+            return;
         }
+        case SLOSH_MODEL_ELASTIC_LINEAR:
+        case SLOSH_MODEL_SAND_LINEAR:
+        case SLOSH_MODEL_SAND_NEO_HOOKEAN:
+            break;
         default:
 #pragma unroll
             for (int i = 0; i < D; ++i)
 #pragma unroll
                 for (int k = 0; k < D; ++k) tau[i][k] = 0.f;
-            break;
+            return;
+    }
+    // sand without a plastic model (its lambda is 0) is purely elastic
+    const bool plastic = tag != SLOSH_MODEL_ELASTIC_LINEAR && mat.p[7] != 0.f;
+    if (tag == SLOSH_MODEL_SAND_NEO_HOOKEAN && !plastic) {
+        neo_hookean<D>(F, mat.p[9], mat.p[10], tau);
+        return;
+    }
+    Stretch<D> b;
+    bool done = b.of(F) && det<D>(F) > 0.f;
+    if (done) {
+        if (!plastic) {
+            const float *el = tag == SLOSH_MODEL_ELASTIC_LINEAR ? mat.p : mat.p + 9;
+            stretch_corotated<D>(b, el[0], el[1], tau);
+        } else if (tag == SLOSH_MODEL_SAND_LINEAR) {
+            done = stretch_sand<D, false>(b, mat.p + 3, mat.p[9], mat.p[10], st, F, tau);
+        } else {
+            done = stretch_sand<D, true>(b, mat.p + 3, mat.p[9], mat.p[10], st, F, tau);
+        }
+    }
+    if (!done) {
+        // through copies, so that F, st and tau themselves stay in registers
+        float Fc[D][D], tc[D][D], sc[3] = {st[0], st[1], st[2]};
+#pragma unroll
+        for (int i = 0; i < D; ++i)
+#pragma unroll
+            for (int k = 0; k < D; ++k) Fc[i][k] = F[i][k];
+        model_update_svd<D>(mat, tag, Fc, sc, tc, fp64);
+#pragma unroll
+        for (int i = 0; i < D; ++i)
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                F[i][k] = Fc[i][k];
+                tau[i][k] = tc[i][k];
+            }
+        st[0] = sc[0];
+        st[1] = sc[1];
+        st[2] = sc[2];
     }
 }
 
