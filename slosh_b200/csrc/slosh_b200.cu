@@ -194,7 +194,7 @@ int nbk(int dim) { return dim == 3 ? Geo<3>::NB : Geo<2>::NB; }
 // round) and P2G takes blocks in rank order (with no more blocks than warps
 // the heaviest-first order balances nothing and its bucket sort is saved).
 constexpr uint32_t G2P_SMALL_PARTICLES = 262144;
-constexpr uint32_t P2G_WIDE_PARTICLES = 1048576;  // P2G in CTAs of six warps below this
+constexpr uint32_t P2G_SHARE_PARTICLES = 1048576;
 
 DevScene make_scene(slosh_ctx *c, uint32_t parity, bool force) {
     DevScene s{};
@@ -284,10 +284,9 @@ DevScene make_scene(slosh_ctx *c, uint32_t parity, bool force) {
     s.use_partial = (c->p2g_variant == 0) ? 1u : 0u;
     s.gather_only = 0u;
     // P2G: one warp a block fills the GPU from about 10 blocks an SM; below
-    // that a CTA's warps share each block.  Scenes below P2G_WIDE_PARTICLES
-    // run CTAs of six warps (3 an SM), which share blocks up to about 5
-    // blocks a CTA (16 an SM): one pass a warp beats six passes a warp there
-    s.p2g_coop_below = c->n < P2G_WIDE_PARTICLES ? (uint32_t)c->sm_count * 16u : (uint32_t)c->sm_count * 10u;
+    // that (16 an SM in a scene of fewer than P2G_SHARE_PARTICLES) four warps
+    // share each block, a pass each
+    s.p2g_coop_below = c->n < P2G_SHARE_PARTICLES ? (uint32_t)c->sm_count * 16u : (uint32_t)c->sm_count * 10u;
     s.p2g_heavy_first = c->n >= G2P_SMALL_PARTICLES ? 1u : 0u;
     s.coll = c->coll[cur];
     s.coll_id = c->coll_id[cur];
@@ -417,17 +416,9 @@ template <int D> void enqueue_p2g(slosh_ctx *c, const DevScene &s, cudaStream_t 
         const uint32_t g = std::min<uint32_t>(c->cap, (uint32_t)c->sm_count * 8);
         launch_k(c, g, P2G_ATOMIC_THREADS, 0, st, k_p2g_atomic<D>, s);
     } else {
-        if (c->n < P2G_WIDE_PARTICLES) {
-            // a small scene: CTAs of six warps, one pass of a shared block each
-            const uint32_t g = std::min<uint32_t>(c->cap, (uint32_t)c->sm_count * 3);
-            constexpr size_t smem = sizeof(P2gSmem<D, 3, P2G_WIDE_WARPS>);
-            if (s.force_pending) launch_k(c, g, 32 * P2G_WIDE_WARPS, smem, st, k_p2g_wide<D, true>, s);
-            else launch_k(c, g, 32 * P2G_WIDE_WARPS, smem, st, k_p2g_wide<D, false>, s);
-        } else {
-            const uint32_t g = std::min<uint32_t>((c->cap + P2G_WARPS - 1) / P2G_WARPS, (uint32_t)c->sm_count * 5);
-            if (s.force_pending) launch_k(c, g, 32 * P2G_WARPS, 0, st, k_p2g<D, false, true>, s);
-            else launch_k(c, g, 32 * P2G_WARPS, 0, st, k_p2g<D>, s);
-        }
+        const uint32_t g = std::min<uint32_t>(c->cap, (uint32_t)c->sm_count * P2G_CTAS_PER_SM);
+        if (s.force_pending) launch_k(c, g, 32 * P2G_WARPS, 0, st, k_p2g<D, false, true>, s);
+        else launch_k(c, g, 32 * P2G_WARPS, 0, st, k_p2g<D>, s);
     }
     PROF_END(12);
 }
@@ -906,15 +897,6 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
         const int v = std::atoi(nt);
         if (v == 64 || v == 128 || v == 256) c->g2p_threads = (uint32_t)v;
     }
-    // the small-scene P2G's shared memory is above the 48 KB a launch gets by default
-    cudaFuncSetAttribute(k_p2g_wide<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(P2gSmem<3, 3, P2G_WIDE_WARPS>));
-    cudaFuncSetAttribute(k_p2g_wide<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(P2gSmem<3, 3, P2G_WIDE_WARPS>));
-    cudaFuncSetAttribute(k_p2g_wide<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(P2gSmem<2, 3, P2G_WIDE_WARPS>));
-    cudaFuncSetAttribute(k_p2g_wide<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(P2gSmem<2, 3, P2G_WIDE_WARPS>));
     if (const char *pdl = std::getenv("SLOSH_PDL")) c->pdl = std::strcmp(pdl, "0") != 0;
     c->reuse_mode = 2u;
     if (const char *r = std::getenv("SLOSH_GRID_REUSE")) c->reuse_mode = std::strcmp(r, "0") == 0 ? 0u : 1u;

@@ -40,403 +40,339 @@ __device__ __forceinline__ bool tile_node_owner(const DevScene &s, uint32_t r, i
     return rank != NONE;
 }
 
-// Adds one particle to a thread's stencil sums.  The thread owns cell `assoc`
-// (its base node, in cells) and one slab of the 3^D stencil: 3D the nodes
-// (sx, sy, slab), 2D (sx, slab).  p = (x, m), vv = (v, C22), cq = C rows,
-// fdt = the pending force impulse (zeros when none).  The weights use
-// -d0 / h = -d0 * (1/h) like slosh's p2g (dpt * inv_cell_width) with
-// d0 = assoc h - x exact from the sorted cell.  Returns false for a
-// particle outside the cell (packed-key aliasing far outside the key range).
+// The quadratic B-spline weights of one axis (kernel.slang:62-68), each
+// duplicated into both lanes of a pair for the paired FMAs below.
+__device__ __forceinline__ void bspline_pairs(float x, float2 (&w)[3]) {
+    const float2 f = pair(x), half = pair(0.5f);
+    const float2 a = __fadd2_rn(pair(1.5f), make_float2(-f.x, -f.y)), b = __fadd2_rn(f, pair(-1.0f)),
+                 c = __fadd2_rn(f, pair(-0.5f));
+    w[0] = __fmul2_rn(__fmul2_rn(half, a), a);
+    w[1] = __ffma2_rn(make_float2(-b.x, -b.y), b, pair(0.75f));
+    w[2] = __fmul2_rn(__fmul2_rn(half, c), c);
+}
+
+// Adds one particle to a lane's stencil sums.  The lane owns cell `assoc`
+// (its base node, in cells) and one half of the node values: half 0 the
+// momentum's (x, y), half 1 (z, mass), (0, mass) in 2D.  p = (x, m), vv = (v,
+// C22), cq = C's planes, fdt = the pending force impulse (zeros when none).
+// The weights use -d0 / h = -d0 * (1/h) like slosh's p2g (dpt *
+// inv_cell_width) with d0 = assoc h - x exact from the sorted cell.  Returns
+// false for a particle outside the cell (packed-key aliasing far outside the
+// key range).
+//
+// Paired FP32 arithmetic (sm_100's f32x2 FMA) throughout: a node's value is
+// b + sx h C0 + sy h C1 + sz h C2 with C's columns restricted to the half
+// (the mass lane's are zero, so it stays m exactly), formed slab by slab and
+// row by row; 27 nodes cost 27 weight products, 26 value and 27 sum pairs.
 template <int D>
 __device__ __forceinline__ bool p2g_particle(const float4 p, const float4 vv, const float4 *cq, const float (&fdt)[3],
-                                             const float (&assoc)[D], float h, float inv_h, int slab,
-                                             float4 (&acc)[D == 3 ? 9 : 3]) {
+                                             const float (&assoc)[D], float h, float inv_h, int half,
+                                             float2 (&acc)[Geo<D>::NST]) {
     const float x[3] = {p.x, p.y, p.z};
-    const float m = p.w;
-    float d0[D], w[D][3], fs = 0.f;
+    float d0[D];
     bool in_cell = true;
+    float2 w[D][3];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
         d0[k] = assoc[k] * h - x[k];
         const float f = -d0[k] * inv_h;
-        in_cell = in_cell && f >= 0.49f && f <= 1.51f;
-        if (k < D - 1) bspline_weights(f, w[k]);
-        else fs = f;
+        in_cell = in_cell && fabsf(f - 1.0f) <= 0.51f;
+        bspline_pairs(f, w[k]);
     }
     if (!in_cell) return false;
-    // Along the slab axis the lane needs its own slab's weight only, in
-    // bspline_weights' arithmetic: (0.5 t) t with t = f - 1.5 (= -(1.5 - f)
-    // exactly) or t = f - 0.5, and 0.75 - t t with t = f - 1.  The
-    // coefficients depend on the slab alone, so they stay out of the loop.
-    const float sb = slab == 0 ? 1.5f : (slab == 1 ? 1.0f : 0.5f);
-    const float sa = slab == 1 ? -1.0f : 0.5f, sc = slab == 1 ? 0.75f : 0.0f;
-    const float ts = fs - sb;
-    const float wsl = fmaf(sa * ts, ts, sc);
-    float bm[D], hc[D][D], Cm[D][D];
-    mat_from<D>(cq, vv.w, Cm);
-    const float vel[3] = {vv.x, vv.y, vv.z};
+    float C[D][D];
+    mat_from<D>(cq, vv.w, C);
+    // columns of C and the base value, restricted to this half
+    float2 col[D], b;
 #pragma unroll
-    for (int jj = 0; jj < D; ++jj) {
-        float q = vel[jj] * m + fdt[jj];
-#pragma unroll
-        for (int k = 0; k < D; ++k) {
-            const float c = Cm[jj][k];
-            q += c * d0[k];
-            hc[k][jj] = h * c;
-        }
-        bm[jj] = q;
+    for (int k = 0; k < D; ++k) {
+        if constexpr (D == 3) col[k] = half ? make_float2(C[2][k], 0.f) : make_float2(C[0][k], C[1][k]);
+        else col[k] = half ? make_float2(0.f, 0.f) : make_float2(C[0][k], C[1][k]);
     }
-    const float fsl = (float)slab;
-    if constexpr (D == 3) {
-        // Paired FP32 arithmetic (sm_100 f32x2 FMA): the node value
-        // (b + s h C, m) is carried as the pairs (x, y) and (z, m); the m
-        // lane's offsets are zero, so it stays m exactly.  Offset 0 adds
-        // nothing to a finite value and is skipped.
-        const float wz = wsl;
-        const float2 hx01 = make_float2(hc[0][0], hc[0][1]), hx2 = make_float2(hc[0][2], 0.f);
-        const float2 hy01 = make_float2(hc[1][0], hc[1][1]), hy2 = make_float2(hc[1][2], 0.f);
-        const float2 fs2 = make_float2(fsl, fsl);
-        const float2 mz01 = __ffma2_rn(fs2, make_float2(hc[2][0], hc[2][1]), make_float2(bm[0], bm[1]));
-        const float2 mz2 = __ffma2_rn(fs2, make_float2(hc[2][2], 0.f), make_float2(bm[2], m));
+    const float m = p.w;
+    if constexpr (D == 3) b = half ? make_float2(vv.z * m + fdt[2], m) : make_float2(vv.x * m + fdt[0], vv.y * m + fdt[1]);
+    else b = half ? make_float2(0.f, m) : make_float2(vv.x * m + fdt[0], vv.y * m + fdt[1]);
+#pragma unroll
+    for (int k = 0; k < D; ++k) b = __ffma2_rn(col[k], pair(d0[k]), b);
+    const float2 h2 = pair(h), two = pair(2.0f);
+#pragma unroll
+    for (int k = 0; k < D; ++k) col[k] = __fmul2_rn(h2, col[k]);
+#pragma unroll
+    for (int sz = 0; sz < (D == 3 ? 3 : 1); ++sz) {
+        float2 bz = b;
+        if constexpr (D == 3) bz = sz == 0 ? b : (sz == 1 ? __fadd2_rn(b, col[2]) : __ffma2_rn(two, col[2], b));
 #pragma unroll
         for (int sy = 0; sy < 3; ++sy) {
-            const float wyz = w[1][sy] * wz;
-            float2 my01 = mz01, my2 = mz2;
-            if (sy > 0) {
-                const float2 sy2 = make_float2((float)sy, (float)sy);
-                my01 = __ffma2_rn(sy2, hy01, mz01);
-                my2 = __ffma2_rn(sy2, hy2, mz2);
-            }
+            const float2 by = sy == 0 ? bz : (sy == 1 ? __fadd2_rn(bz, col[1]) : __ffma2_rn(two, col[1], bz));
+            float2 wyz = w[1][sy];
+            if constexpr (D == 3) wyz = __fmul2_rn(w[1][sy], w[2][sz]);
 #pragma unroll
             for (int sx = 0; sx < 3; ++sx) {
-                float2 t01 = my01, t2 = my2;
-                if (sx > 0) {
-                    const float2 sx2 = make_float2((float)sx, (float)sx);
-                    t01 = __ffma2_rn(sx2, hx01, my01);
-                    t2 = __ffma2_rn(sx2, hx2, my2);
-                }
-                const float wt = w[0][sx] * wyz;
-                const float2 wt2 = make_float2(wt, wt);
-                float4 &a = acc[sx + 3 * sy];
-                const float2 axy = __ffma2_rn(wt2, t01, make_float2(a.x, a.y));
-                const float2 azw = __ffma2_rn(wt2, t2, make_float2(a.z, a.w));
-                a = make_float4(axy.x, axy.y, azw.x, azw.y);
+                const float2 v = sx == 0 ? by : (sx == 1 ? __fadd2_rn(by, col[0]) : __ffma2_rn(two, col[0], by));
+                float2 &a = acc[sx + 3 * (sy + 3 * sz)];
+                a = __ffma2_rn(__fmul2_rn(w[0][sx], wyz), v, a);
             }
-        }
-    } else {
-        const float wy = wsl;
-        const float my0 = bm[0] + fsl * hc[1][0], my1 = bm[1] + fsl * hc[1][1];
-#pragma unroll
-        for (int sx = 0; sx < 3; ++sx) {
-            const float wt = w[0][sx] * wy;
-            float4 &a = acc[sx];
-            a.x += wt * (my0 + (float)sx * hc[0][0]);
-            a.y += wt * (my1 + (float)sx * hc[0][1]);
-            a.w += wt * m;
         }
     }
     return true;
 }
 
-// Particle-to-grid, one warp per active block (P2G_WARPS warps a CTA, each
-// on its own blocks, no CTA barrier).
+// Particle-to-grid over the blocks of the sorted grid.
 //
-// The block's 64 cells x 3 stencil slabs are 192 (cell, slab) items, taken
-// in bord's order (cells by decreasing particle count) in 6 passes of 32:
-// the lanes of a pass hold cells of similar count, so they finish their
+// A block's 64 cells x 2 halves of the node values are 128 items, taken in
+// bord's order (cells by decreasing particle count) in 4 passes of 32: the
+// lanes of a pass hold 16 cells of similar count, so they finish their
 // particle loops together, and a pass whose first (largest) cell is empty
-// ends the block.  A lane owns cell c and the 9 (3D) or 3 (2D) stencil nodes
-// of one slab, reads the particles of c -- contiguous in the canonical order
-// -- double-buffered through cp.async, and sums its nodes in registers.
+// ends the block.  A lane owns cell c, sums the c's particles -- contiguous
+// in the canonical order, staged NBUF deep through cp.async, the two lanes of
+// a cell copying half of the particle each -- into its 27 (9) stencil nodes'
+// half values in registers.
 //
-// Reduction, fixed order (the substep is bit-reproducible): each slab has a
-// tile of the nodes its cells reach (3D: 6 x 6 x 4, z relative to the slab;
-// 2D: 10 x 8).  After each pass the lanes add their 9 (3) sums, one stencil
-// offset at a time; for a fixed offset the lanes of a pass hit distinct
-// nodes (one item per (cell, slab)), so only __syncwarp is needed.  The
-// slab tiles are then summed in slab order into the block's (block + 2)^D
-// tile, stored to its own `partial` slot; k_grid_update adds the (up to 2^D)
-// tiles overlapping each node in a fixed order.
-constexpr int P2G_WARPS = 4;
-template <int D> struct SlabTile;
-template <> struct SlabTile<3> {
-    static constexpr int PY = 6, PZ = 36, SIZE = 144;  // x 6, y 6, z 4
-};
-template <> struct SlabTile<2> {
-    static constexpr int PY = 10, PZ = 0, SIZE = 80;  // x 10, y 8
-};
-
+// Why halves: every lane of a cell computes the particle's weights and base
+// value again, so fewer lanes a cell means less of that; a whole node value a
+// lane (108 sums) does not fit the registers.  With three z slabs a cell
+// (nine nodes, whole values) the same sums took a third more instructions and
+// the block three slab tiles (measured on the 4.74 M sand column: P2G_OLD
+// against P2G_NEW us a launch).
+//
+// Reduction, fixed order (the substep is bit-reproducible): after a pass the
+// lanes add their sums into the warp's (block + 2)^D tile, one stencil offset
+// at a time; for a fixed offset the lanes of a pass hit distinct node halves,
+// so only __syncwarp is needed.  With a block per warp the passes follow each
+// other on one tile; where a group of warps shares a block (small scenes) the
+// warps' tiles are summed in warp order.  The tile goes to the block's own
+// `partial` slot; k_grid_update adds the (up to 2^D) tiles overlapping each
+// node in a fixed order.
+//
 // FORCE: the substep adds the particles' pending force impulses (the first
 // substep after they were set); the other substeps compile without them.
 // NBUF: particles of a cell staged ahead through cp.async (batches tune it;
 // the results do not depend on it).
-// Shared memory of k_p2g's CTA (P2G_WARPS warps): each warp's three slab
-// tiles and its staged particles.  Staging: the particles of a pass's cells
-// (at most CS = 12: 32 lanes, 3 slab lanes a cell, the first and last cell
-// possibly shared with the neighbouring passes) in NBUF buffers; particle
-// k + NBUF - 1 of every cell is copied while particle k is summed.
+constexpr int P2G_WARPS = 4;
+constexpr uint32_t P2G_PASSES = 4;
+template <int D, int NBUF> struct P2gWarp {
+    float4 tile[Geo<D>::TILE];
+    float4 pm[NBUF][16], vv[NBUF][16], cq[NBUF][MQ<D>::Q][16];
+};
+// Shared memory of W warps (one group).
 template <int D, int NBUF, int W = P2G_WARPS> struct P2gSmem {
-    static constexpr int CS = 12;
-    float4 stile[W][3 * SlabTile<D>::SIZE];
-    float4 sp_pm[W][NBUF][CS];
-    float4 sp_vv[W][NBUF][CS];
-    float4 sp_cq[W][NBUF][MQ<D>::Q][CS];
+    P2gWarp<D, NBUF> w[W];
 };
 
-template <int D, bool B = false, bool FORCE = false, int NBUF = 3, int W = P2G_WARPS>
-__device__ __forceinline__ void p2g_body(const DevScene &s, P2gSmem<D, NBUF, W> &sm) {
-    constexpr int TW = Geo<D>::TW, TILE = Geo<D>::TILE, BW = Geo<D>::BW;
-    constexpr int NACC = (D == 3) ? 9 : 3;
-    constexpr int PY = SlabTile<D>::PY, PZ = SlabTile<D>::PZ, SSZ = SlabTile<D>::SIZE;
+// One pass of block r: 32 (cell, half) items (`ord` their cells) summed into
+// the warp's tile.  Returns false when the pass's cells are empty (and so are
+// the later passes').  With `next`, `ord` is reloaded with the next pass's
+// cells once this pass's are read.  `src`: storage index of the block's first
+// particle when its particles are one shifted range of storage, else NONE
+// (the permutation is read).
+template <int D, bool FORCE, int NBUF>
+__device__ __forceinline__ bool p2g_pass(const DevScene &s, P2gWarp<D, NBUF> &wm, uint32_t r, uint32_t first,
+                                         uint32_t src, const int (&bv)[D], float h, float inv_h, uint32_t pass,
+                                         uint2 &ord, bool next) {
+    constexpr int TW = Geo<D>::TW, BW = Geo<D>::BW, NST = Geo<D>::NST;
     constexpr int Q = MQ<D>::Q;
-    constexpr int CS = P2gSmem<D, NBUF, W>::CS;
     static_assert(NBUF >= 2 && NBUF <= 4, "staging depth 2 to 4");
-    auto &stile = sm.stile;
-    auto &sp_pm = sm.sp_pm;
-    auto &sp_vv = sm.sp_vv;
-    auto &sp_cq = sm.sp_cq;
-    // storage index of the current block's first particle when its
-    // particles are one shifted range of storage, else NONE (the
-    // permutation is read)
-    uint32_t src = NONE;
-    const bool use_src = !B && s.reuse && s.bsrc != nullptr;
-    const uint32_t nb = s.ctr->n_blocks;
+    const uint32_t lane = lane_id();
     const size_t n = s.n;
-    const uint32_t lane = lane_id(), wl = threadIdx.x >> 5;
-    float4 *tiles = stile[wl];
-    // One pass of block r: 32 (cell, slab) items (`ord` their cells)
-    // summed into this warp's slab tiles.  Returns false when the pass's
-    // cells are empty (and so are the later passes').  With `next`, `ord`
-    // is reloaded with the next pass's cells once this pass's are read.
-    auto run_pass = [&](uint32_t r, uint32_t first, const int (&bv)[D], float h, float inv_h, uint32_t pass,
-                        uint2 &ord, bool next) -> bool {
-        const uint32_t item = 32u * pass + lane;
-        const int slab = (int)(item % 3u);
-        const uint32_t lo = ord.x >> 6, hi = lo + ord.y;
-        const int cell = (int)(ord.x & 63u);
-        if (__shfl_sync(FULL_MASK, ord.y, 0) == 0u) return false;
-        if (next) ord = s.bord[(size_t)r * CELLS + (item + 32u) / 3u];
-        int ca[D];
-        if constexpr (D == 3) {
-            ca[0] = cell & 3;
-            ca[1] = (cell >> 2) & 3;
-            ca[2] = cell >> 4;
-        } else {
-            ca[0] = cell & 7;
-            ca[1] = cell >> 3;
-        }
-        float assoc[D];
+    const int half = (int)(lane & 1u);
+    const uint32_t cs = lane >> 1;  // the cell's staging slot
+    const uint32_t lo = ord.x >> 6, cnt = ord.y;
+    const int cell = (int)(ord.x & 63u);
+    const uint32_t kmax = __shfl_sync(FULL_MASK, cnt, 0);
+    if (kmax == 0u) return false;
+    if (next) ord = s.bord[(size_t)r * CELLS + 16u * (pass + 1u) + cs];
+    int ca[D];
+    if constexpr (D == 3) {
+        ca[0] = cell & 3;
+        ca[1] = (cell >> 2) & 3;
+        ca[2] = cell >> 4;
+    } else {
+        ca[0] = cell & 7;
+        ca[1] = cell >> 3;
+    }
+    float assoc[D];
 #pragma unroll
-        for (int k = 0; k < D; ++k) assoc[k] = (float)(bv[k] * BW + ca[k]);
-        float4 acc[NACC];
+    for (int k = 0; k < D; ++k) assoc[k] = (float)(bv[k] * BW + ca[k]);
+    float2 acc[NST];
 #pragma unroll
-        for (int k = 0; k < NACC; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        // The first lane of each cell in this pass (its slab-0 lane, or lane
-        // 0 for a cell begun in the previous pass) copies the cell's
-        // particles into the cell's staging slot; the three slab lanes of a
-        // cell read the same slot.  The lanes step through particle k
-        // together (k up to the pass's largest count, lane 0's), so the warp
-        // can sync around the copies.
-        const uint32_t cnt = hi - lo, kmax = __shfl_sync(FULL_MASK, cnt, 0);
-        const uint32_t cs = item / 3u - (32u * pass) / 3u;
-        const bool loader = slab == 0 || lane == 0;
-        auto stage = [&](uint32_t k, uint32_t i) {
-            if (loader && k < cnt) {
-                const int b = (int)(k % NBUF);
-                cp_async16(&sp_pm[wl][b][cs], &s.pm[i]);
-                cp_async16(&sp_vv[wl][b][cs], &s.vv[i]);
+    for (int k = 0; k < NST; ++k) acc[k] = make_float2(0.f, 0.f);
+    // the lanes step through particle k together (k up to the pass's largest
+    // count, lane 0's), so the warp can sync around the copies
+    auto stage = [&](uint32_t k, uint32_t i) {
+        if (k < cnt) {
+            const int b = (int)(k % NBUF);
+            if (half == 0) {
+                cp_async16(&wm.pm[b][cs], &s.pm[i]);
+                cp_async16(&wm.vv[b][cs], &s.vv[i]);
+            } else {
 #pragma unroll
-                for (int q = 0; q < Q; ++q) cp_async16(&sp_cq[wl][b][q][cs], &s.cq[q * n + i]);
+                for (int q = 0; q < Q; ++q) cp_async16(&wm.cq[b][q][cs], &s.cq[q * n + i]);
             }
-            cp_async_commit();
-        };
-        auto index = [&](uint32_t k) {
-            return (loader && k < cnt) ? (src != NONE ? src + lo + k : s.perm[first + lo + k]) : 0u;
-        };
-#pragma unroll
-        for (uint32_t k = 0; k + 1 < (uint32_t)NBUF; ++k) stage(k, index(k));
-        uint32_t i_next = index(NBUF - 1u);  // loaded one iteration before its copies
-        for (uint32_t k = 0; k < kmax; ++k) {
-            stage(k + NBUF - 1u, i_next);
-            i_next = index(k + NBUF);
-            cp_async_wait<NBUF - 1>();
-            __syncwarp();  // the loaders' copies of particle k have landed
-            if (k < cnt) {
-                const int b = (int)(k % NBUF);
-                float fdt[3] = {0.f, 0.f, 0.f};
-                if constexpr (FORCE) {
-                    const uint32_t i = src != NONE ? src + lo + k : s.perm[first + lo + k];
-#pragma unroll
-                    for (int d = 0; d < D; ++d) fdt[d] = s.fdt[d * n + i];
-                }
-                float4 cv[Q];
-#pragma unroll
-                for (int q = 0; q < Q; ++q) cv[q] = sp_cq[wl][b][q][cs];
-                if (!p2g_particle<D>(sp_pm[wl][b][cs], sp_vv[wl][b][cs], cv, fdt, assoc, h, inv_h, slab, acc))
-                    atomicOr(s.err, ERR_KEY_RANGE);
-            }
-            __syncwarp();  // slot k % NBUF is refilled by the next iteration's copies
         }
-        cp_async_wait<0>();
+        cp_async_commit();
+    };
+    auto index = [&](uint32_t k) { return k < cnt ? (src != NONE ? src + lo + k : s.perm[first + lo + k]) : 0u; };
+#pragma unroll
+    for (uint32_t k = 0; k + 1 < (uint32_t)NBUF; ++k) stage(k, index(k));
+    uint32_t i_next = index(NBUF - 1u);  // loaded one iteration before its copies
+    for (uint32_t k = 0; k < kmax; ++k) {
+        stage(k + NBUF - 1u, i_next);
+        i_next = index(k + NBUF);
+        cp_async_wait<NBUF - 1>();
+        __syncwarp();  // both lanes' copies of particle k have landed
+        if (k < cnt) {
+            const int b = (int)(k % NBUF);
+            float fdt[3] = {0.f, 0.f, 0.f};
+            if constexpr (FORCE) {
+                const uint32_t i = src != NONE ? src + lo + k : s.perm[first + lo + k];
+#pragma unroll
+                for (int d = 0; d < D; ++d) fdt[d] = s.fdt[d * n + i];
+            }
+            float4 cv[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) cv[q] = wm.cq[b][q][cs];
+            if (!p2g_particle<D>(wm.pm[b][cs], wm.vv[b][cs], cv, fdt, assoc, h, inv_h, half, acc))
+                atomicOr(s.err, ERR_KEY_RANGE);
+        }
+        __syncwarp();  // slot k % NBUF is refilled by the next iteration's copies
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    float2 *pt = reinterpret_cast<float2 *>(wm.tile) + half;
+    int base = ca[0] + TW * ca[1];
+    if constexpr (D == 3) base += TW * TW * ca[2];
+#pragma unroll
+    for (int k = 0; k < NST; ++k) {
+        const int idx = base + k % 3 + TW * ((k / 3) % 3) + TW * TW * (k / 9);
+        pt[2 * idx] = __fadd2_rn(pt[2 * idx], acc[k]);
         __syncwarp();
-        // node (cell + stencil offset) in the slab's tile, whose slab-axis
-        // coordinate is relative to the slab: 3D z - slab = ca[2], 2D
-        // y - slab = ca[1]
-        float4 *pt = tiles + slab * SSZ;
-#pragma unroll
-        for (int k = 0; k < NACC; ++k) {
-            const int sx = k % 3;
-            int idx;
-            if constexpr (D == 3) idx = (ca[0] + sx) + PY * (ca[1] + k / 3) + PZ * ca[2];
-            else idx = (ca[0] + sx) + PY * ca[1];
-            float4 v = pt[idx];
-            v.x += acc[k].x;
-            v.y += acc[k].y;
-            v.z += acc[k].z;
-            v.w += acc[k].w;
-            pt[idx] = v;
-            __syncwarp();
+    }
+    return true;
+}
+
+// The block of rank r as P2G needs it: cell width, cell origin, first entry.
+// False for a block without particles, or with stale counts (left by an
+// earlier overflow).
+template <int D, bool B> struct P2gBlock {
+    float h, inv_h;
+    int bv[D];
+    uint32_t first, src;
+    __device__ __forceinline__ bool load(const DevScene &s, uint32_t r, bool report) {
+        const uint32_t np = s.bnp[r];
+        if (np == 0) return false;
+        first = s.bfirst[r];
+        if ((size_t)first + np > s.n) {
+            if (report) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
+            return false;
         }
-        return true;
-    };
-    // Node t of the block's (block + 2)^D tile: the sum of the slab tiles of
-    // warps [w0, w1) in warp then slab order.
-    auto tile_node = [&](int t, uint32_t w0, uint32_t w1) {
-        int tc[D];
-        tc[0] = t % TW;
-        if constexpr (D == 3) {
-            tc[1] = (t / TW) % TW;
-            tc[2] = t / (TW * TW);
-        } else {
-            tc[1] = t / TW;
-        }
-        const int along = tc[D - 1];  // slab axis: z in 3D, y in 2D
-        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (uint32_t w = w0; w < w1; ++w)
-#pragma unroll
-            for (int sl = 0; sl < 3; ++sl) {
-                const int rel = along - sl;  // node plane within slab sl's tile
-                if (rel < 0 || rel >= BW) continue;
-                const int lay = (D == 3) ? tc[0] + PY * tc[1] + PZ * rel : tc[0] + PY * rel;
-                const float4 v = stile[w][sl * SSZ + lay];
-                sum.x += v.x;
-                sum.y += v.y;
-                sum.z += v.z;
-                sum.w += v.w;
-            }
-        return sum;
-    };
-    auto block_setup = [&](uint32_t r, float &h, float &inv_h, int (&bv)[D]) {
-        if constexpr (B) {
-            h = s.scenes[s.bscene[r]].h;
-            inv_h = 1.0f / h;
-        }
+        h = s.h;
+        if constexpr (B) h = s.scenes[s.bscene[r]].h;
+        inv_h = 1.0f / h;
         unpack_key<D>(s.bkey[r], bv);
-        for (uint32_t q = lane; q < 3u * SSZ; q += 32u) tiles[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        src = (!B && s.reuse && s.bsrc != nullptr) ? s.bsrc[r] : NONE;
+        return true;
+    }
+};
+template <int D, int NBUF> __device__ __forceinline__ void p2g_zero_tile(P2gWarp<D, NBUF> &wm) {
+    for (int q = (int)lane_id(); q < Geo<D>::TILE; q += 32) wm.tile[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+}
+
+// Block r by one warp.
+template <int D, bool B, bool FORCE, int NBUF>
+__device__ __forceinline__ void p2g_warp_block(const DevScene &s, P2gWarp<D, NBUF> &wm, uint32_t r) {
+    P2gBlock<D, B> k;
+    if (!k.load(s, r, lane_id() == 0)) return;
+    p2g_zero_tile<D>(wm);
+    uint2 ord = s.bord[(size_t)r * CELLS + (lane_id() >> 1)];
+    for (uint32_t pass = 0; pass < P2G_PASSES; ++pass)
+        if (!p2g_pass<D, FORCE>(s, wm, r, k.first, k.src, k.bv, k.h, k.inv_h, pass, ord, pass + 1u < P2G_PASSES)) break;
+    __syncwarp();
+    for (int t = (int)lane_id(); t < Geo<D>::TILE; t += 32) s.partial[(size_t)r * Geo<D>::TILE + t] = wm.tile[t];
+    __syncwarp();
+}
+
+// Block r by a group of P2G_WARPS warps, a pass each; thread `t` of the
+// group, which `sync` synchronises.
+template <int D, bool FORCE, int NBUF, typename Sync>
+__device__ __forceinline__ void p2g_group_block(const DevScene &s, P2gSmem<D, NBUF> &sm, uint32_t r, uint32_t t,
+                                                Sync sync) {
+    constexpr int TILE = Geo<D>::TILE;
+    static_assert(P2G_WARPS == P2G_PASSES, "a pass a warp");
+    const uint32_t wl = t >> 5;
+    P2gBlock<D, false> k;
+    if (!k.load(s, r, t == 0)) return;  // the same for the whole group
+    p2g_zero_tile<D>(sm.w[wl]);
+    uint2 ord = s.bord[(size_t)r * CELLS + 16u * wl + (lane_id() >> 1)];
+    p2g_pass<D, FORCE>(s, sm.w[wl], r, k.first, k.src, k.bv, k.h, k.inv_h, wl, ord, false);
+    sync();
+    for (int q = (int)t; q < TILE; q += 32 * P2G_WARPS) {
+        float4 sum = sm.w[0].tile[q];
+#pragma unroll
+        for (int w = 1; w < P2G_WARPS; ++w) {
+            const float4 v = sm.w[w].tile[q];
+            sum.x += v.x;
+            sum.y += v.y;
+            sum.z += v.z;
+            sum.w += v.w;
+        }
+        s.partial[(size_t)r * TILE + q] = sum;
+    }
+    sync();  // the tiles are zeroed for the next block
+}
+
+template <int D, bool B = false, bool FORCE = false, int NBUF = 3>
+__device__ __forceinline__ void p2g_body(const DevScene &s, P2gSmem<D, NBUF> &sm) {
+    const uint32_t nb = s.ctr->n_blocks;
+    // blocks are taken from a queue (one atomic a block), so warps that get
+    // light blocks take more of them
+    auto next = [&]() {
+        const uint32_t q = atomicAdd(&s.ctr->p2g_next, 1u);
+        return q < nb ? (s.p2g_heavy_first ? s.qorder[q] : q) : nb;
     };
-    if (!B && nb < s.p2g_coop_below) {
-        // Few blocks (a small scene): the CTA's W warps share a block, warp w
-        // taking passes w, w + W, ..., and the block's tile sums the warps'
-        // slab tiles in warp order.
+    if (!B && nb < s.p2g_coop_below) {  // few blocks (a small scene): the CTA's warps share a block
         __shared__ uint32_t coop_r;
         for (;;) {
-            __syncthreads();  // the previous block's tile sum has read the slab tiles
-            if (threadIdx.x == 0) {
-                const uint32_t q = atomicAdd(&s.ctr->p2g_next, 1u);
-                coop_r = q < nb ? (s.p2g_heavy_first ? s.qorder[q] : q) : nb;
-            }
+            __syncthreads();
+            if (threadIdx.x == 0) coop_r = next();
             __syncthreads();
             const uint32_t r = coop_r;
-            if (r >= nb) break;
-            const uint32_t np = s.bnp[r];
-            if (np == 0) continue;
-            const uint32_t first = s.bfirst[r];
-            if (first + np > s.n) {
-                if (threadIdx.x == 0) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
-                continue;
-            }
-            float h = s.h, inv_h = 1.0f / s.h;
-            int bv[D];
-            block_setup(r, h, inv_h, bv);
-            src = use_src ? s.bsrc[r] : NONE;
-            for (uint32_t pass = wl; pass < 6u; pass += W) {
-                uint2 ord = s.bord[(size_t)r * CELLS + (32u * pass + lane) / 3u];
-                if (!run_pass(r, first, bv, h, inv_h, pass, ord, false)) break;
-            }
-            __syncthreads();
-            for (int t = (int)threadIdx.x; t < TILE; t += 32 * W)
-                s.partial[(size_t)r * TILE + t] = tile_node(t, 0, W);
+            if (r >= nb) return;
+            p2g_group_block<D, FORCE>(s, sm, r, threadIdx.x, [] { __syncthreads(); });
         }
-        return;
     }
-    // One warp a block.  Blocks are taken from a queue (one atomic a
-    // block), so warps that get light blocks take more of them.
-    auto next_block = [&]() {
+    for (;;) {
         uint32_t r = 0;
-        if (lane == 0) {
-            const uint32_t q = atomicAdd(&s.ctr->p2g_next, 1u);
-            r = q < nb ? (s.p2g_heavy_first ? s.qorder[q] : q) : nb;
-        }
-        return __shfl_sync(FULL_MASK, r, 0);
-    };
-    for (uint32_t r = next_block(); r < nb; r = next_block()) {
-        const uint32_t np = s.bnp[r];
-        if (np == 0) continue;
-        const uint32_t first = s.bfirst[r];
-        if (first + np > s.n) {  // only after an earlier overflow left stale counts
-            if (lane == 0) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
-            continue;
-        }
-        float h = s.h, inv_h = 1.0f / s.h;
-        int bv[D];
-        block_setup(r, h, inv_h, bv);
-        src = use_src ? s.bsrc[r] : NONE;
-        uint2 ord = s.bord[(size_t)r * CELLS + lane / 3u];
-        for (uint32_t pass = 0; pass < 6u; ++pass)
-            if (!run_pass(r, first, bv, h, inv_h, pass, ord, pass < 5u)) break;  // later passes hold empty cells
-        __syncwarp();
-        for (int t = (int)lane; t < TILE; t += 32) s.partial[(size_t)r * TILE + t] = tile_node(t, wl, wl + 1);
-        __syncwarp();
+        if (lane_id() == 0) r = next();
+        r = __shfl_sync(FULL_MASK, r, 0);
+        if (r >= nb) return;
+        p2g_warp_block<D, B, FORCE>(s, sm.w[threadIdx.x >> 5], r);
     }
 }
+constexpr int P2G_CTAS_PER_SM = 4;
 template <int D, bool B = false, bool FORCE = false, int NBUF = 3>
-__global__ void __launch_bounds__(32 * P2G_WARPS, 5) k_p2g(DevScene s) {
+__global__ void __launch_bounds__(32 * P2G_WARPS, P2G_CTAS_PER_SM) k_p2g(DevScene s) {
     pdl_enter();
     __shared__ P2gSmem<D, NBUF> sm;
     p2g_body<D, B, FORCE, NBUF>(s, sm);
 }
 
-// Small scenes: CTAs of P2G_WIDE_WARPS warps, which take one pass each of a
-// shared block (3 CTAs an SM by registers); their shared memory (54 KB in
-// 3D) is dynamic.
-constexpr int P2G_WIDE_WARPS = 6;
-template <int D, bool FORCE>
-__global__ void __launch_bounds__(32 * P2G_WIDE_WARPS, 3) k_p2g_wide(DevScene s) {
-    pdl_enter();
-    extern __shared__ __align__(16) unsigned char psm[];
-    p2g_body<D, false, FORCE, 3, P2G_WIDE_WARPS>(s, *reinterpret_cast<P2gSmem<D, 3, P2G_WIDE_WARPS> *>(psm));
-}
-
 // Particle-to-grid with float atomics, kept for comparison (SLOSH_P2G=direct):
-// one CTA of 192 threads a block, thread (cell, slab) sums its nodes like
+// one CTA of 128 threads a block, thread (cell, half) sums its nodes like
 // k_p2g and adds them through shared-memory atomics into the block's tile,
 // then 16-byte global atomics into the nodes.  Not bit-reproducible.
-constexpr int P2G_ATOMIC_THREADS = 192;
+constexpr int P2G_ATOMIC_THREADS = 128;
 template <int D> __global__ void __launch_bounds__(P2G_ATOMIC_THREADS, 4) k_p2g_atomic(DevScene s) {
     pdl_enter();
-    constexpr int TW = Geo<D>::TW, TILE = Geo<D>::TILE, BW = Geo<D>::BW;
-    constexpr int NACC = (D == 3) ? 9 : 3;
+    constexpr int TW = Geo<D>::TW, TILE = Geo<D>::TILE, BW = Geo<D>::BW, NST = Geo<D>::NST;
     constexpr int NT = P2G_ATOMIC_THREADS;
     constexpr int Q = MQ<D>::Q;
-    __shared__ float tile[4][TILE];
-    __shared__ float4 sp_pm[2][NT];
-    __shared__ float4 sp_vv[2][NT];
-    __shared__ float4 sp_cq[2][Q][NT];
+    __shared__ float4 tile[TILE];
     const uint32_t nb = s.ctr->n_blocks;
     const float h = s.h, inv_h = 1.0f / s.h;
     const size_t n = s.n;
     const uint32_t tid = threadIdx.x;
-    const int mycell = (int)(tid & 63u), myslab = (int)(tid >> 6);
+    const int mycell = (int)(tid >> 1), half = (int)(tid & 1u);
     int ca[D];
     if constexpr (D == 3) {
         ca[0] = mycell & 3;
@@ -454,7 +390,7 @@ template <int D> __global__ void __launch_bounds__(P2G_ATOMIC_THREADS, 4) k_p2g_
             if (tid == 0) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
             continue;
         }
-        for (int t = tid; t < 4 * TILE; t += NT) (&tile[0][0])[t] = 0.f;
+        for (int t = tid; t < TILE; t += NT) tile[t] = make_float4(0.f, 0.f, 0.f, 0.f);
         int bv[D];
         unpack_key<D>(s.bkey[r], bv);
         const uint32_t lo = s.bcell[(size_t)r * CELLS + mycell];
@@ -462,53 +398,36 @@ template <int D> __global__ void __launch_bounds__(P2G_ATOMIC_THREADS, 4) k_p2g_
         float assoc[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) assoc[k] = (float)(bv[k] * BW + ca[k]);
-        float4 acc[NACC];
+        float2 acc[NST];
 #pragma unroll
-        for (int k = 0; k < NACC; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        auto stage = [&](int b, uint32_t j) {
-            if (j < hi) {
-                const uint32_t i = s.perm[first + j];
-                cp_async16(&sp_pm[b][tid], &s.pm[i]);
-                cp_async16(&sp_vv[b][tid], &s.vv[i]);
-#pragma unroll
-                for (int q = 0; q < Q; ++q) cp_async16(&sp_cq[b][q][tid], &s.cq[q * n + i]);
-            }
-            cp_async_commit();
-        };
-        stage(0, lo);
+        for (int k = 0; k < NST; ++k) acc[k] = make_float2(0.f, 0.f);
         __syncthreads();
-        int buf = 0;
-        for (uint32_t j = lo; j < hi; ++j, buf ^= 1) {
-            stage(buf ^ 1, j + 1);
-            cp_async_wait<1>();
+        for (uint32_t j = lo; j < hi; ++j) {
+            const uint32_t i = s.perm[first + j];
             float fdt[3] = {0.f, 0.f, 0.f};
             if (s.force_pending) {
-                const uint32_t i = s.perm[first + j];
 #pragma unroll
                 for (int k = 0; k < D; ++k) fdt[k] = s.fdt[k * n + i];
             }
             float4 cv[Q];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) cv[q] = sp_cq[buf][q][tid];
-            if (!p2g_particle<D>(sp_pm[buf][tid], sp_vv[buf][tid], cv, fdt, assoc, h, inv_h, myslab, acc))
-                atomicOr(s.err, ERR_KEY_RANGE);
+            for (int q = 0; q < Q; ++q) cv[q] = s.cq[q * n + i];
+            if (!p2g_particle<D>(s.pm[i], s.vv[i], cv, fdt, assoc, h, inv_h, half, acc)) atomicOr(s.err, ERR_KEY_RANGE);
         }
-        cp_async_wait<0>();
         if (hi > lo) {
+            float *pt = reinterpret_cast<float *>(tile) + 2 * half;
+            int base = ca[0] + TW * ca[1];
+            if constexpr (D == 3) base += TW * TW * ca[2];
 #pragma unroll
-            for (int k = 0; k < NACC; ++k) {
-                const int sx = k % 3, sy = (D == 3) ? k / 3 : myslab, sz = (D == 3) ? myslab : 0;
-                int idx = (ca[0] + sx) + TW * (ca[1] + sy);
-                if constexpr (D == 3) idx += TW * TW * (ca[2] + sz);
-                atomicAdd(&tile[0][idx], acc[k].x);
-                atomicAdd(&tile[1][idx], acc[k].y);
-                if constexpr (D == 3) atomicAdd(&tile[2][idx], acc[k].z);
-                atomicAdd(&tile[3][idx], acc[k].w);
+            for (int k = 0; k < NST; ++k) {
+                const int idx = base + k % 3 + TW * ((k / 3) % 3) + TW * TW * (k / 9);
+                atomicAdd(&pt[4 * idx], acc[k].x);
+                atomicAdd(&pt[4 * idx + 1], acc[k].y);
             }
         }
         __syncthreads();
         for (int t = tid; t < TILE; t += NT) {
-            const float4 val = make_float4(tile[0][t], tile[1][t], tile[2][t], tile[3][t]);
+            const float4 val = tile[t];
             if (val.x == 0.f && val.y == 0.f && val.z == 0.f && val.w == 0.f) continue;
             uint32_t rank, local;
             if (!tile_node_owner<D>(s, r, t, rank, local)) continue;
