@@ -230,12 +230,16 @@ class ClockSampler:
 def timed_launches(data, st0: dict, st1: dict, steps: int):
     """Kernels launched by `steps` substeps between two stats snapshots, and
     how many of them kept their grid: with conditional graphs a substep that
-    keeps its grid launches 7 kernels fewer than one that rebuilds it."""
+    keeps its grid launches 7 kernels fewer than one that rebuilds it, and a
+    small scene's substeps (one kernel a substep reported) share launches of up
+    to 32."""
     reused = st1["n_grid_reuses"] - st0["n_grid_reuses"]
     rebuilt = st1["n_grid_rebuilds"] - st0["n_grid_rebuilds"]
     full = data.kernels_per_substep
     if st1["conditional_graphs"]:
         launches = full * rebuilt + (full - 7) * reused
+    elif full == 1:
+        launches = -(-steps // 32)
     else:
         launches = data.kernels_per_substep * steps
     return launches, {"reused_substeps": reused, "rebuilt_substeps": rebuilt,

@@ -246,8 +246,9 @@ int slosh_add_trimesh(slosh_ctx *ctx, const float *vertices, uint32_t n_vertices
  * hold particles, and only re-counts the cells particles entered or left;
  * the decision is taken on the device.  The layout is the one a full build
  * gives, bit for bit.  Scenes of at least 262,144 particles keep their grid
- * this way; smaller ones are launch-bound, and the full build inside the
- * substep graph is faster for them.  The environment variable
+ * this way; below 180,000 in 3D (262,144 in 2D) up to 32 substeps, each with
+ * the full build, run as one cooperative launch (the same bits; SLOSH_SCENE_STEPS=0 at context
+ * creation keeps the separate kernels).  The environment variable
  * SLOSH_GRID_REUSE at context creation overrides that: 0 makes every
  * substep run the full build, 1 keeps grids at any size. */
 int slosh_step(slosh_ctx *ctx, uint32_t n_substeps, void *stream);
@@ -331,7 +332,8 @@ int slosh_sync(slosh_ctx *ctx, void *stream);
  * build (for launch accounting).  With grid reuse and conditional graphs a
  * substep that keeps the previous grid launches 7 fewer: the reuse's
  * permutation update and touched-cell gather instead of the 9 build
- * kernels (slosh_get_stats counts both kinds of substep). */
+ * kernels (slosh_get_stats counts both kinds of substep).  1: the scene's
+ * substeps share launches of up to 32. */
 uint32_t slosh_kernels_per_substep(const slosh_ctx *ctx);
 
 /* Runs `n_substeps` substeps with direct launches (not the CUDA graph) and a

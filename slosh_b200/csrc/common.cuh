@@ -29,7 +29,7 @@ constexpr uint32_t ERR_KEY_RANGE = 1u << 4;        // a block coordinate outside
 constexpr uint32_t ERR_BLOCK_PARTICLES = 1u << 6;  // a block holds 2^26 particles or more
 constexpr uint32_t ERR_SCENE_BLOCKS = 1u << 5;     // a batch scene has more blocks than the per-scene sort holds
 constexpr uint32_t ERR_GRID_REUSE = 1u << 7;       // a kept grid's cell counts and its gathered cells disagree
-constexpr uint32_t ERR_BARRIER = 1u << 8;          // a grid barrier of the fused batch substep gave up waiting
+constexpr uint32_t ERR_BARRIER = 1u << 8;          // a grid barrier gave up waiting
 
 // Sparse grid geometry per dimension (shaders/slosh/grid/grid.slang:224-257).
 template <int D> struct Geo;
@@ -329,7 +329,8 @@ struct Counters {
     uint32_t n_touched;      // touched cells listed by k_reuse_perm for k_reuse_cells
     uint32_t bar_count;      // fused batch substep: CTAs arrived at the current grid barrier
     uint32_t bar_gen;        // fused batch substep: grid barriers completed (wraps)
-    uint32_t pad[2];
+    uint32_t steps_ticket;   // k_scene_steps: barrier arrivals of the running launch
+    uint32_t steps_left;     // k_scene_steps: CTAs that left the running launch
 };
 
 // The CTA index and CTA count a kernel body runs with: its own launch's

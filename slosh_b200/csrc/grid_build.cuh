@@ -142,8 +142,11 @@ template <bool B = false> __global__ void k_clear(DevScene s) {
     }
     if constexpr (B)
         for (uint32_t i = tid; i < s.n_scenes; i += stride) s.scene_nblk[i] = 0u;
-    if (*s.err != 0u)
+    if (*s.err != 0u) {
         for (size_t i = tid; i < (size_t)s.hcap * CELLS; i += stride) s.slot_counts[i] = 0u;
+        if (!B && s.slot_total)
+            for (uint32_t i = tid; i < s.hcap; i += stride) s.slot_total[i] = 0u;
+    }
     for (uint32_t i = tid; i < HIST_BINS; i += stride) s.hist[i] = 0u;
     if (tid < HIST_COARSE) s.hist_coarse[tid] = 0u;
     if (tid == 0) {
@@ -566,9 +569,74 @@ __global__ void k_scene_rank(DevScene s) { pdl_enter(); scene_rank_body(s, launc
 // neighbour ranks (update_nbh_block_ids, sort.slang:100-117), the block's
 // rank in the previous substep's map (the grid update's collision cache) and, for the
 // atomic P2G variants, zeroed nodes (reset, grid.slang:455-485).
+//
+// block_cells: the cells of the block with hash slot `sl` and rank r (the
+// whole warp); returns the block's particle count.
+__device__ __forceinline__ uint32_t block_cells(const DevScene &s, uint32_t r, uint32_t sl) {
+    const uint32_t lane = lane_id();
+    uint2 *cnt = reinterpret_cast<uint2 *>(s.slot_counts + ((size_t)sl << 6));
+    const uint2 c = cnt[lane];
+    cnt[lane] = make_uint2(0u, 0u);
+    const uint32_t c0 = c.x, c1 = c.y, both = c0 + c1;
+    uint32_t incl = both;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL_MASK, incl, off);
+        if (lane >= (uint32_t)off) incl += y;
+    }
+    const uint32_t ex = incl - both;
+    const uint2 firsts = make_uint2(ex, ex + c0);
+    reinterpret_cast<uint2 *>(s.bcell + (size_t)r * CELLS)[lane] = firsts;
+    reinterpret_cast<uint2 *>(s.bcur + (size_t)r * CELLS)[lane] = firsts;
+    const uint32_t total = __shfl_sync(FULL_MASK, incl, 31);
+    if (lane == 31) {
+        s.bnp[r] = total;
+        if (total >= (1u << 26)) atomicOr(s.err, ERR_BLOCK_PARTICLES);  // beyond the 26-bit first in bord
+        if (s.bsrc) s.bsrc[r] = NONE;  // a full build's permutation is no shifted range
+    }
+    // rank of each cell among the 64 by (count desc, cell asc): the number
+    // of keys above its own, keys being distinct
+    const uint32_t k0 = (min(c0, 0x3ffffffu) << 6) | (63u - 2u * lane);
+    const uint32_t k1 = (min(c1, 0x3ffffffu) << 6) | (62u - 2u * lane);
+    uint32_t r0 = 0, r1 = 0;
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) {
+        const uint32_t a = __shfl_sync(FULL_MASK, k0, q), b = __shfl_sync(FULL_MASK, k1, q);
+        r0 += (a > k0) + (b > k0);
+        r1 += (a > k1) + (b > k1);
+    }
+    s.bord[(size_t)r * CELLS + r0] = make_uint2((2u * lane) | (ex << 6), c0);
+    s.bord[(size_t)r * CELLS + r1] = make_uint2((2u * lane + 1u) | ((ex + c0) << 6), c1);
+    return total;
+}
+
+// block_neighbors: the +1 and -1 neighbours' ranks and the block's previous
+// rank, once every block has its rank in the map.
+template <int D, bool B> __device__ __forceinline__ void block_neighbors(const DevScene &s, uint32_t r) {
+    constexpr int NN = Geo<D>::NASSOC - 1;
+    const uint32_t lane = lane_id();
+    // lanes [0, NN): the +1 neighbours b + o; lanes [NN, 2 NN): the -1
+    // neighbours b - o, whose P2G tiles overlap this block.
+    if (lane < (uint32_t)(2 * NN)) {
+        const bool fwd = lane < (uint32_t)NN;
+        const int q = fwd ? (int)lane : (int)lane - NN;
+        int b[D], o[D];
+        unpack_key<D>(s.bkey[r], b);
+        assoc_offset<D>(q + 1, o);
+        for (int k = 0; k < D; ++k) b[k] += fwd ? o[k] : -o[k];
+        const uint32_t slot = map_find<B>(s, pack_key<D>(b), B ? s.bscene[r] : 0u);
+        const uint32_t v = (slot == NONE) ? NONE : s.hvals[slot];
+        // the grid update gathers the tiles of the -1 neighbours that hold particles
+        if (fwd) s.bnbh[r * NN + q] = rank_of(v);
+        else s.bnbh_rev[r * NN + q] = (v & RANK_EXTRA) ? NONE : v;
+    } else if (lane == (uint32_t)(2 * NN)) {
+        const uint32_t slot = map_find_prev<B>(s, s.bkey[r], B ? s.bscene[r] : 0u);
+        s.bprev[r] = (slot == NONE) ? NONE : rank_of(s.prev_hvals[slot]);
+    }
+}
+
 template <int D, bool B = false> __device__ __forceinline__ void block_setup_body(const DevScene &s, Cta g) {
     if (build_skipped(s)) return;  // this substep keeps the previous grid
-    constexpr int NN = Geo<D>::NASSOC - 1;
     const uint32_t nb = s.ctr->n_blocks;
     const uint32_t lane = lane_id();
     const uint32_t warps = g.n * (blockDim.x >> 5);
@@ -580,70 +648,17 @@ template <int D, bool B = false> __device__ __forceinline__ void block_setup_bod
                 for (uint32_t c = 0; c < G2P_CLASSES; ++c) s.g2p_counts[G2P_CLASSES + c] = 0u;
     }
     for (uint32_t r = g.id * (blockDim.x >> 5) + (threadIdx.x >> 5); r < nb; r += warps) {
-        const uint32_t sl = s.bslot[r];
-        uint32_t *cnt = s.slot_counts + ((size_t)sl << 6);
-        const uint32_t c0 = cnt[2 * lane], c1 = cnt[2 * lane + 1];
-        cnt[2 * lane] = 0u;
-        cnt[2 * lane + 1] = 0u;
-        const uint32_t pair = c0 + c1;
-        uint32_t incl = pair;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(FULL_MASK, incl, off);
-            if (lane >= (uint32_t)off) incl += y;
-        }
-        const uint32_t ex = incl - pair;
-        s.bcell[(size_t)r * CELLS + 2 * lane] = ex;
-        s.bcell[(size_t)r * CELLS + 2 * lane + 1] = ex + c0;
-        s.bcur[(size_t)r * CELLS + 2 * lane] = ex;
-        s.bcur[(size_t)r * CELLS + 2 * lane + 1] = ex + c0;
-        if (lane == 31) {
-            s.bnp[r] = incl;
-            if (incl >= (1u << 26)) atomicOr(s.err, ERR_BLOCK_PARTICLES);  // beyond the 26-bit first in bord
-            if (s.bsrc) s.bsrc[r] = NONE;  // a full build's permutation is no shifted range
-            if constexpr (B)
-                if (s.g2p_lists && incl != 0u) {  // the block goes to its scene's G2P launch
-                    const uint32_t cls = s.scenes[s.bscene[r]].g2p_class;
-                    s.g2p_lists[(size_t)cls * s.cap + atomicAdd(&s.g2p_counts[cls], 1u)] = r;
-                }
-        }
-        {
-            // rank of each cell among the 64 by (count desc, cell asc): the
-            // number of keys above its own, keys being distinct
-            const uint32_t k0 = (min(c0, 0x3ffffffu) << 6) | (63u - 2u * lane);
-            const uint32_t k1 = (min(c1, 0x3ffffffu) << 6) | (62u - 2u * lane);
-            uint32_t r0 = 0, r1 = 0;
-#pragma unroll 8
-            for (int q = 0; q < 32; ++q) {
-                const uint32_t a = __shfl_sync(FULL_MASK, k0, q), b = __shfl_sync(FULL_MASK, k1, q);
-                r0 += (a > k0) + (b > k0);
-                r1 += (a > k1) + (b > k1);
+        const uint32_t np = block_cells(s, r, s.bslot[r]);
+        if constexpr (B)
+            if (lane == 0 && s.g2p_lists && np != 0u) {  // the block goes to its scene's G2P launch
+                const uint32_t cls = s.scenes[s.bscene[r]].g2p_class;
+                s.g2p_lists[(size_t)cls * s.cap + atomicAdd(&s.g2p_counts[cls], 1u)] = r;
             }
-            s.bord[(size_t)r * CELLS + r0] = make_uint2((2u * lane) | (ex << 6), c0);
-            s.bord[(size_t)r * CELLS + r1] = make_uint2((2u * lane + 1u) | ((ex + c0) << 6), c1);
-        }
         if (!s.use_partial) {  // the atomic P2G variants accumulate into the nodes
             s.nodes[(size_t)r * 64 + 2 * lane] = make_float4(0.f, 0.f, 0.f, 0.f);
             s.nodes[(size_t)r * 64 + 2 * lane + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        // lanes [0, NN): the +1 neighbours b + o; lanes [NN, 2 NN): the -1
-        // neighbours b - o, whose P2G tiles overlap this block.
-        if (lane < (uint32_t)(2 * NN)) {
-            const bool fwd = lane < (uint32_t)NN;
-            const int q = fwd ? (int)lane : (int)lane - NN;
-            int b[D], o[D];
-            unpack_key<D>(s.bkey[r], b);
-            assoc_offset<D>(q + 1, o);
-            for (int k = 0; k < D; ++k) b[k] += fwd ? o[k] : -o[k];
-            const uint32_t slot = map_find<B>(s, pack_key<D>(b), B ? s.bscene[r] : 0u);
-            const uint32_t v = (slot == NONE) ? NONE : s.hvals[slot];
-            // the grid update gathers the tiles of the -1 neighbours that hold particles
-            if (fwd) s.bnbh[r * NN + q] = rank_of(v);
-            else s.bnbh_rev[r * NN + q] = (v & RANK_EXTRA) ? NONE : v;
-        } else if (lane == (uint32_t)(2 * NN)) {
-            const uint32_t slot = map_find_prev<B>(s, s.bkey[r], B ? s.bscene[r] : 0u);
-            s.bprev[r] = (slot == NONE) ? NONE : rank_of(s.prev_hvals[slot]);
-        }
+        block_neighbors<D, B>(s, r);
     }
 }
 template <int D, bool B = false> __global__ void k_block_setup(DevScene s) {
@@ -778,67 +793,68 @@ __device__ __forceinline__ void sort_cell_keys(unsigned long long *key, uint32_t
     }
 }
 
+// canon_block: warp `part` of the `G` that share block r sorts the cells c
+// with c % G == part (cells are disjoint, so the result does not depend on G).
+__device__ __forceinline__ void canon_block(const DevScene &s, uint32_t r, uint32_t part, uint32_t G) {
+    const uint32_t lane = lane_id();
+    const uint32_t first = s.bfirst[r], np = s.bnp[r];
+    if (np < 2) return;
+    if ((size_t)first + np > s.n) {  // only after an earlier overflow left stale counts
+        if (lane == 0 && part == 0) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
+        return;
+    }
+    const unsigned long long *k = s.skey + first;
+    unsigned long long bad = 0ull;  // cells holding an inversion
+    for (uint32_t e = lane; e + 1 < np; e += 32) {
+        const unsigned long long k0 = k[e], k1 = k[e + 1];
+        if (k0 > k1 && (k0 >> 32) == (k1 >> 32)) bad |= 1ull << (uint32_t)(k0 >> 32);
+    }
+    if (G > 1u) {
+        unsigned long long mine = 0ull;
+        for (uint32_t c = part; c < CELLS; c += G) mine |= 1ull << c;
+        bad &= mine;
+    }
+    const uint32_t lo = __reduce_or_sync(FULL_MASK, (uint32_t)bad);
+    const uint32_t hi = __reduce_or_sync(FULL_MASK, (uint32_t)(bad >> 32));
+    if ((lo | hi) == 0u) return;
+    unsigned long long cells = ((unsigned long long)hi << 32) | lo;
+    while (cells != 0ull) {
+        const uint32_t c = (uint32_t)__ffsll((long long)cells) - 1u;
+        cells &= cells - 1ull;
+        const uint32_t b0 = s.bcell[(size_t)r * CELLS + c];
+        const uint32_t b1 = (c < CELLS - 1) ? s.bcell[(size_t)r * CELLS + c + 1] : np;
+        if (b1 <= b0 + 1 || b1 > np) continue;
+        const uint32_t m = b1 - b0;
+        unsigned long long *ck = s.skey + first + b0;
+        uint32_t *cp = s.perm + first + b0;
+        if (m > 32u) {
+            if (lane == 0) sort_cell_keys(ck, cp, m);
+            __syncwarp();
+            continue;
+        }
+        const unsigned long long kl = lane < m ? ck[lane] : ~0ull;
+        const uint32_t pl = lane < m ? cp[lane] : 0u;
+        const uint32_t id = (uint32_t)kl;  // the cell part of the keys is equal
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < m; ++j) rank += __shfl_sync(FULL_MASK, id, j) < id ? 1u : 0u;
+        __syncwarp();  // every lane has read its entry
+        if (lane < m) {
+            ck[rank] = kl;
+            cp[rank] = pl;
+        }
+        __syncwarp();
+    }
+}
+
 __device__ __forceinline__ void canon_body(const DevScene &s, Cta g) {
     if (build_skipped(s)) return;  // this substep keeps the previous grid
     const uint32_t nb = s.ctr->n_blocks;
-    const uint32_t lane = lane_id();
     const uint32_t warps = g.n * (blockDim.x >> 5);
-    // With few blocks (a small scene) G warps share a block, warp `part`
-    // sorting the cells c with c % G == part, so that a block's out-of-order
-    // cells are sorted side by side instead of one after another.  Cells
-    // are disjoint, so the result does not depend on G.
+    // With few blocks (a small scene) G warps share a block, so that its
+    // out-of-order cells are sorted side by side instead of one after another.
     uint32_t G = 1u;
     while (G < 8u && (size_t)nb * G * 2u <= warps) G <<= 1;
-    for (uint32_t t = g.id * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nb * G; t += warps) {
-        const uint32_t r = t / G, part = t % G;
-        const uint32_t first = s.bfirst[r], np = s.bnp[r];
-        if (np < 2) continue;
-        if ((size_t)first + np > s.n) {  // only after an earlier overflow left stale counts
-            if (lane == 0 && part == 0) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
-            continue;
-        }
-        const unsigned long long *k = s.skey + first;
-        unsigned long long bad = 0ull;  // cells holding an inversion
-        for (uint32_t e = lane; e + 1 < np; e += 32) {
-            const unsigned long long k0 = k[e], k1 = k[e + 1];
-            if (k0 > k1 && (k0 >> 32) == (k1 >> 32)) bad |= 1ull << (uint32_t)(k0 >> 32);
-        }
-        if (G > 1u) {
-            unsigned long long mine = 0ull;
-            for (uint32_t c = part; c < CELLS; c += G) mine |= 1ull << c;
-            bad &= mine;
-        }
-        const uint32_t lo = __reduce_or_sync(FULL_MASK, (uint32_t)bad);
-        const uint32_t hi = __reduce_or_sync(FULL_MASK, (uint32_t)(bad >> 32));
-        if ((lo | hi) == 0u) continue;
-        unsigned long long cells = ((unsigned long long)hi << 32) | lo;
-        while (cells != 0ull) {
-            const uint32_t c = (uint32_t)__ffsll((long long)cells) - 1u;
-            cells &= cells - 1ull;
-            const uint32_t b0 = s.bcell[(size_t)r * CELLS + c];
-            const uint32_t b1 = (c < CELLS - 1) ? s.bcell[(size_t)r * CELLS + c + 1] : np;
-            if (b1 <= b0 + 1 || b1 > np) continue;
-            const uint32_t m = b1 - b0;
-            unsigned long long *ck = s.skey + first + b0;
-            uint32_t *cp = s.perm + first + b0;
-            if (m > 32u) {
-                if (lane == 0) sort_cell_keys(ck, cp, m);
-                __syncwarp();
-                continue;
-            }
-            const unsigned long long kl = lane < m ? ck[lane] : ~0ull;
-            const uint32_t pl = lane < m ? cp[lane] : 0u;
-            const uint32_t id = (uint32_t)kl;  // the cell part of the keys is equal
-            uint32_t rank = 0;
-            for (uint32_t j = 0; j < m; ++j) rank += __shfl_sync(FULL_MASK, id, j) < id ? 1u : 0u;
-            __syncwarp();  // every lane has read its entry
-            if (lane < m) {
-                ck[rank] = kl;
-                cp[rank] = pl;
-            }
-            __syncwarp();
-        }
-    }
+    for (uint32_t t = g.id * (blockDim.x >> 5) + (threadIdx.x >> 5); t < nb * G; t += warps) canon_block(s, t / G, t % G, G);
 }
 __global__ void k_canon(DevScene s) { pdl_enter(); canon_body(s, launch_cta()); }
 

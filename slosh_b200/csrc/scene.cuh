@@ -49,6 +49,8 @@ struct DevScene {
     uint32_t *clr_hvals;
     uint32_t clear_tail;
     uint32_t *slot_counts; // hcap * 64 per-cell particle counts per hash slot
+    uint32_t *slot_total;  // hcap particle counts per hash slot (scene_step.cuh; null in batches)
+    uint2 *items;          // k_scene_steps: 32-particle parts of blocks, (block, part) or (NONE, -)
     uint32_t *blist_key;   // primary blocks in append order [cap]
     uint32_t *blist_slot;
     uint32_t *blist2_key;  // neighbour-only blocks in append order [cap]
@@ -127,9 +129,9 @@ struct DevScene {
     uint32_t *scene_nblk;            // blocks per scene this substep
     uint32_t *scene_bbase;           // first block rank of each scene
     uint32_t *scene_fill;            // scatter cursors
-    // fused substep's grid barrier: arrivals expected beyond the launch's
-    // CTAs (0; a test sets more to make the wait run out) and its time
-    // limit in ns (0: the default)
+    // grid barriers of the one-launch substeps (batch, small scene):
+    // arrivals expected beyond the launch's CTAs (0; a test sets more to make
+    // the wait run out) and the time limit in ns (0: the default)
     uint32_t bar_extra;
     unsigned long long bar_ns;
     // G2P by scene class: the blocks of each class (G2P_CLASSES lists of

@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <thread>
 #include <vector>
 
@@ -20,6 +21,7 @@
 #include "transfer.cuh"
 #include "timestep.cuh"
 #include "fused.cuh"
+#include "scene_step.cuh"
 
 using namespace slosh;
 
@@ -47,11 +49,11 @@ struct slosh_ctx {
 
     // grid
     uint32_t *hkeys[2] = {nullptr, nullptr}, *hvals[2] = {nullptr, nullptr};
-    uint32_t *slot_counts = nullptr, *blist_key = nullptr, *blist_slot = nullptr, *blist2_key = nullptr,
+    uint32_t *slot_counts = nullptr, *slot_total = nullptr, *blist_key = nullptr, *blist_slot = nullptr, *blist2_key = nullptr,
              *blist2_slot = nullptr, *hist = nullptr, *hist_start = nullptr, *hist_coarse = nullptr, *tmp_key = nullptr,
              *tmp_slot = nullptr, *bkey = nullptr, *bslot = nullptr, *bfirst = nullptr, *bnp = nullptr,
              *bcell = nullptr, *bcur = nullptr, *bnbh = nullptr, *bnbh_rev = nullptr;
-    uint2 *bord = nullptr;
+    uint2 *bord = nullptr, *items = nullptr;
     uint32_t *qorder = nullptr, *bprev = nullptr;
     // grid reuse (single-scene contexts): the second parity's block arrays
     // and G2P's per-cell bookkeeping; reuse = 0 in batches and when the
@@ -81,6 +83,12 @@ struct slosh_ctx {
     // turns it off).  pdl_capture: a substep graph is being captured;
     // pdl_link: the previous operation captured on the stream is a kernel.
     bool pdl = true, pdl_capture = false, pdl_link = false;
+    // Substeps of a small scene as one cooperative launch (SLOSH_SCENE_STEPS=0
+    // turns it off; also off where the device cannot hold it).
+    bool scene_steps = true;
+    // SLOSH_FUSED_BARRIER_TEST="<extra arrivals>:<limit ns>", as for a batch
+    uint32_t bar_extra = 0;
+    unsigned long long bar_ns = 0;
     uint32_t *pslot = nullptr, *perm = nullptr;
     unsigned long long *skey = nullptr;
     float4 *nodes = nullptr, *partial = nullptr, *coll[2] = {nullptr, nullptr};
@@ -236,6 +244,8 @@ DevScene make_scene(slosh_ctx *c, uint32_t parity, bool force) {
     s.prev_hkeys = c->hkeys[prv];
     s.prev_hvals = c->hvals[prv];
     s.slot_counts = c->slot_counts;
+    s.slot_total = c->slot_total;
+    s.items = c->items;
     s.blist_key = c->blist_key;
     s.blist_slot = c->blist_slot;
     s.blist2_key = c->blist2_key;
@@ -283,6 +293,8 @@ DevScene make_scene(slosh_ctx *c, uint32_t parity, bool force) {
     s.partial = c->partial;
     s.use_partial = (c->p2g_variant == 0) ? 1u : 0u;
     s.gather_only = 0u;
+    s.bar_extra = c->bar_extra;
+    s.bar_ns = c->bar_ns;
     // P2G: one warp a block fills the GPU from about 10 blocks an SM; below
     // that (16 an SM in a scene of fewer than P2G_SHARE_PARTICLES) four warps
     // share each block, a pass each
@@ -508,6 +520,80 @@ constexpr uint32_t REUSE_MIN_PARTICLES = 262144;
 
 void destroy_graphs(slosh_ctx *c);
 
+// ---- a small scene's substeps in one launch (scene_step.cuh) ----------------
+// Below this many particles a substep is bound by the latency of its stages
+// and by their launches; above it one CTA of 512 threads an SM runs P2G and G2P
+// slower than their own kernels do.  Microseconds a substep, one launch
+// against separate kernels: 3D blobs of 30 k fluid particles 40 and 58, 97 k 56
+// and 66, 149 k 65 and 71, 195 k 76 and 75, 250 k 95 and 82 (sand the same
+// order); 2D dam breaks of 63 k 32 and 51, 154 k 54 and 61, 251 k 62 and 72.
+constexpr uint32_t STEPS_MAX_PARTICLES_3D = 180000, STEPS_MAX_PARTICLES_2D = 262144;
+// Substeps a launch takes at most, so that no launch holds the GPU for long.
+constexpr uint32_t STEPS_PER_LAUNCH = 32;
+
+bool takes_scene_steps(const slosh_ctx *c) {
+    return c->scene_steps && !c->reuse && c->p2g_variant == 0 &&
+           c->n < (c->dim == 3 ? STEPS_MAX_PARTICLES_3D : STEPS_MAX_PARTICLES_2D);
+}
+
+template <int D, bool POW2, int MODEL>
+cudaError_t launch_scene_steps(slosh_ctx *c, const ScenePair &pair, uint32_t n, cudaStream_t st) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((uint32_t)c->sm_count);
+    cfg.blockDim = dim3(STEPS_THREADS);
+    cfg.dynamicSmemBytes = sizeof(StepsSmem<D>);
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_scene_steps<D, POW2, MODEL>, pair, c->parity, n);
+}
+// The kernel's instantiations for dimension D, as launch_g2p chooses them.
+template <int D, typename Fn> auto with_scene_steps(const slosh_ctx *c, bool pow2, Fn fn) {
+    if (!pow2) return fn(std::integral_constant<bool, false>(), std::integral_constant<int, -1>());
+    const std::integral_constant<bool, true> yes;
+    if (c->model_mask == 1u << SLOSH_MODEL_SAND_LINEAR) return fn(yes, std::integral_constant<int, SLOSH_MODEL_SAND_LINEAR>());
+    if (c->model_mask == 1u << SLOSH_MODEL_ELASTIC_LINEAR)
+        return fn(yes, std::integral_constant<int, SLOSH_MODEL_ELASTIC_LINEAR>());
+    if (c->model_mask == 1u << SLOSH_MODEL_FLUID_TAIT) return fn(yes, std::integral_constant<int, SLOSH_MODEL_FLUID_TAIT>());
+    return fn(yes, std::integral_constant<int, -1>());
+}
+template <int D> cudaError_t enqueue_scene_steps_d(slosh_ctx *c, uint32_t n, cudaStream_t st) {
+    ScenePair pair;
+    pair.s[0] = make_scene(c, 0, false);
+    pair.s[1] = make_scene(c, 1, false);
+    return with_scene_steps<D>(c, pair.s[0].h_pow2 != 0u, [&](auto pow2, auto model) {
+        return launch_scene_steps<D, decltype(pow2)::value, decltype(model)::value>(c, pair, n, st);
+    });
+}
+cudaError_t enqueue_scene_steps(slosh_ctx *c, uint32_t n, cudaStream_t st) {
+    return c->dim == 3 ? enqueue_scene_steps_d<3>(c, n, st) : enqueue_scene_steps_d<2>(c, n, st);
+}
+
+// Prepares the kernels of dimension D; false when the device cannot hold a
+// cooperative launch of one CTA an SM.
+template <int D> bool scene_steps_fit(const slosh_ctx *c) {
+    bool ok = true;
+    auto one = [&](auto pow2, auto model) {
+        auto *k = k_scene_steps<D, decltype(pow2)::value, decltype(model)::value>;
+        int per_sm = 0;
+        ok = ok &&
+             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepsSmem<D>)) == cudaSuccess &&
+             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, STEPS_THREADS, sizeof(StepsSmem<D>)) == cudaSuccess &&
+             per_sm >= 1;
+    };
+    const std::integral_constant<bool, true> yes;
+    one(std::integral_constant<bool, false>(), std::integral_constant<int, -1>());
+    one(yes, std::integral_constant<int, -1>());
+    one(yes, std::integral_constant<int, SLOSH_MODEL_SAND_LINEAR>());
+    one(yes, std::integral_constant<int, SLOSH_MODEL_ELASTIC_LINEAR>());
+    one(yes, std::integral_constant<int, SLOSH_MODEL_FLUID_TAIT>());
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
 // Sets whether substeps keep their grid, from the mode and the particle
 // count; the graphs are rebuilt when that changes.
 void update_reuse(slosh_ctx *c) {
@@ -713,6 +799,16 @@ int check_device_error(slosh_ctx *c) {
     uint32_t e = 0;
     CK(cudaMemcpy(&e, c->err, 4, cudaMemcpyDeviceToHost));
     if (e == 0) return SLOSH_OK;
+    if ((e & ERR_BARRIER) && c->slot_total) {
+        // k_scene_steps left in the middle of a substep: both maps and the
+        // counts are cleared (while the error is set), the barrier restarts
+        for (uint32_t par = 0; par < 2; ++par)
+            k_clear<false><<<(uint32_t)c->sm_count * 4, 256, 0, c->stream>>>(make_scene(c, par, false));
+        CK(cudaStreamSynchronize(c->stream));
+        CK(cudaMemset(&c->ctr->steps_ticket, 0, 2 * sizeof(uint32_t)));
+        CK(cudaMemset(c->err, 0, 4));
+        return fail(c, SLOSH_E_TIMEOUT, "a grid barrier of the scene's substeps gave up waiting (error bits 0x%x)", e);
+    }
     CK(cudaMemset(c->err, 0, 4));
     if (e & (ERR_HASH_OVERFLOW | ERR_BLOCK_OVERFLOW))
         return fail(c, SLOSH_E_OVERFLOW, "active blocks exceed the grid capacity %u (error bits 0x%x)", c->cap, e);
@@ -879,7 +975,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
         (st = dalloc(c, &c->staging, N)) || (st = dalloc(c, &c->bfirst2, cap)) || (st = dalloc(c, &c->bnp2, cap)) ||
         (st = dalloc(c, &c->bcell2, (size_t)cap * CELLS)) || (st = dalloc(c, &c->cell_delta, (size_t)cap * CELLS)) ||
         (st = dalloc(c, &c->touch, cap)) || (st = dalloc(c, &c->cur_touch, cap)) ||
-        (st = dalloc(c, &c->reuse_cta, 2 * (size_t)REUSE_MAX_CTAS)) ||
+        (st = dalloc(c, &c->slot_total, hcap)) || (st = dalloc(c, &c->items, N / 32 + cap + 1)) || (st = dalloc(c, &c->reuse_cta, 2 * (size_t)REUSE_MAX_CTAS)) ||
         (st = dalloc(c, &c->touched_cells, (size_t)cap * CELLS)) || (st = dalloc(c, &c->bsrc, cap)))
         return fail_create(st);
     cudaMemset(c->hkeys[0], 0xff, hcap * 4);
@@ -889,6 +985,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
     cudaMemset(c->ctr, 0, sizeof(Counters));
     cudaMemset(c->err, 0, 4);
     cudaMemset(c->slot_counts, 0, (size_t)hcap * CELLS * 4);
+    cudaMemset(c->slot_total, 0, (size_t)hcap * 4);
     cudaMemset(c->body_imp, 0, (size_t)MAX_BODIES * 6 * sizeof(unsigned long long));
     if (const char *variant = std::getenv("SLOSH_P2G")) {
         if (std::strcmp(variant, "direct") == 0) c->p2g_variant = 3;
@@ -898,6 +995,19 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
         if (v == 64 || v == 128 || v == 256) c->g2p_threads = (uint32_t)v;
     }
     if (const char *pdl = std::getenv("SLOSH_PDL")) c->pdl = std::strcmp(pdl, "0") != 0;
+    if (const char *v = std::getenv("SLOSH_SCENE_STEPS")) c->scene_steps = std::strcmp(v, "0") != 0;
+    if (const char *bt = std::getenv("SLOSH_FUSED_BARRIER_TEST")) {
+        unsigned extra = 0;
+        unsigned long long ns = 0;
+        if (std::sscanf(bt, "%u:%llu", &extra, &ns) == 2) {
+            c->bar_extra = extra;
+            c->bar_ns = ns;
+        }
+    }
+    int coop = 0;
+    c->scene_steps = c->scene_steps &&
+                     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop &&
+                     (D == 3 ? scene_steps_fit<3>(c) : scene_steps_fit<2>(c));
     c->reuse_mode = 2u;
     if (const char *r = std::getenv("SLOSH_GRID_REUSE")) c->reuse_mode = std::strcmp(r, "0") == 0 ? 0u : 1u;
     update_reuse(c);
@@ -949,6 +1059,7 @@ int slosh_upload_particles(slosh_ctx *c, const slosh_particle *particles, uint32
         CK(cudaMemsetAsync(c->hvals[k], 0xff, c->hcap * 4, st));
     }
     CK(cudaMemsetAsync(c->slot_counts, 0, (size_t)c->hcap * CELLS * 4, st));
+    CK(cudaMemsetAsync(c->slot_total, 0, (size_t)c->hcap * 4, st));
     CK(cudaMemsetAsync(c->hist, 0, HIST_BINS * 4, st));
     CK(cudaMemsetAsync(c->hist_coarse, 0, HIST_COARSE * 4, st));
     c->parity = 0;
@@ -1182,6 +1293,19 @@ int slosh_step(slosh_ctx *c, uint32_t n_substeps, void *stream) {
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     for (uint32_t k = 0; k < n_substeps; ++k) {
+        if (!c->n_hooks && !c->force_pending && takes_scene_steps(c)) {
+            // like the graphs, not part of a stream capture
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            CK(cudaStreamIsCapturing(st, &cap));
+            if (cap != cudaStreamCaptureStatusNone)
+                return fail(c, SLOSH_E_CUDA, "substeps cannot be captured: %s",
+                            cudaGetErrorString(cudaErrorStreamCaptureUnsupported));
+            const uint32_t m = std::min(n_substeps - k, STEPS_PER_LAUNCH);
+            CK(enqueue_scene_steps(c, m, st));
+            c->parity ^= m & 1u;
+            k += m - 1u;
+            continue;
+        }
         if (c->n_hooks) {
             const int r = c->dim == 3 ? enqueue_substep_hooked<3>(c, st, c->parity, c->force_pending != 0)
                                       : enqueue_substep_hooked<2>(c, st, c->parity, c->force_pending != 0);
@@ -1281,6 +1405,7 @@ int slosh_sync(slosh_ctx *c, void *stream) {
 
 uint32_t slosh_kernels_per_substep(const slosh_ctx *c) {
     if (!c) return 0;
+    if (takes_scene_steps(c)) return 1u;  // one launch covers up to STEPS_PER_LAUNCH substeps
     // the full build's 9 kernels, P2G, the grid update, G2P and the rigid
     // update; with grid reuse the decision, and without conditional graphs
     // also the two reuse kernels, which return at once in a full build

@@ -206,13 +206,13 @@ __device__ __forceinline__ void stretch_corotated(const Stretch<D> &b, float lam
         const float sg = sqrtf(1.f + b.m);  // sqrt(b) = sg sqrt(I + X)
         float c0, c1, c2;
         matrix_horner(poly_sqrt(), b.X.p, b.X.q, c0, c1, c2);
-        const float k0 = b.m * __fdividef(sg, 1.f + sg) - sg * c0;
+        const float k0 = fmaf(b.m, __fdividef(sg, 1.f + sg), -(sg * c0));
         const float k1 = fmaf(-sg, c1, 1.f + b.m), k2 = -sg * c2;
         b.X.combine(fmaf(mu2, k0, iso), mu2 * k1, mu2 * k2, tau);
     } else {
         // closed form: sqrt(b) = (b + J I) / t, t^2 = tr b + 2 J
         const float t2 = fmaf(2.f, b.m, 2.f + 2.f * J), t = sqrtf(t2), it = __fdividef(1.f, t);
-        const float det_e = b.m * b.m - (1.f + b.m) * (1.f + b.m) * b.X.p;  // det(b - I)
+        const float det_e = fmaf(b.m, b.m, -((1.f + b.m) * (1.f + b.m) * b.X.p));  // det(b - I)
         const float ke = 1.f - it, k0 = -det_e * __fdividef(it, t + 1.f + J);
         // E = m I + (1 + m) X
         b.X.combine(fmaf(mu2, fmaf(ke, b.m, k0), iso), mu2 * (ke * (1.f + b.m)), 0.f, tau);

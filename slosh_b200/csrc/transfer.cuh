@@ -74,7 +74,7 @@ __device__ __forceinline__ bool p2g_particle(const float4 p, const float4 vv, co
     float2 w[D][3];
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        d0[k] = assoc[k] * h - x[k];
+        d0[k] = fmaf(assoc[k], h, -x[k]);
         const float f = -d0[k] * inv_h;
         in_cell = in_cell && fabsf(f - 1.0f) <= 0.51f;
         bspline_pairs(f, w[k]);
@@ -164,14 +164,14 @@ template <int D, int NBUF, int W = P2G_WARPS> struct P2gSmem {
 // the later passes').  With `next`, `ord` is reloaded with the next pass's
 // cells once this pass's are read.  `src`: storage index of the block's first
 // particle when its particles are one shifted range of storage, else NONE
-// (the permutation is read).
+// (`perm`, the block's part of the permutation, is read).
 template <int D, bool FORCE, int NBUF>
-__device__ __forceinline__ bool p2g_pass(const DevScene &s, P2gWarp<D, NBUF> &wm, uint32_t r, uint32_t first,
+__device__ __forceinline__ bool p2g_pass(const DevScene &s, P2gWarp<D, NBUF> &wm, uint32_t r, const uint32_t *perm,
                                          uint32_t src, const int (&bv)[D], float h, float inv_h, uint32_t pass,
                                          uint2 &ord, bool next) {
     constexpr int TW = Geo<D>::TW, BW = Geo<D>::BW, NST = Geo<D>::NST;
     constexpr int Q = MQ<D>::Q;
-    static_assert(NBUF >= 2 && NBUF <= 4, "staging depth 2 to 4");
+    static_assert(NBUF >= 2, "at least two staged particles");
     const uint32_t lane = lane_id();
     const size_t n = s.n;
     const int half = (int)(lane & 1u);
@@ -198,9 +198,8 @@ __device__ __forceinline__ bool p2g_pass(const DevScene &s, P2gWarp<D, NBUF> &wm
     for (int k = 0; k < NST; ++k) acc[k] = make_float2(0.f, 0.f);
     // the lanes step through particle k together (k up to the pass's largest
     // count, lane 0's), so the warp can sync around the copies
-    auto stage = [&](uint32_t k, uint32_t i) {
+    auto stage = [&](uint32_t k, int b, uint32_t i) {  // particle k into buffer b = k mod NBUF
         if (k < cnt) {
-            const int b = (int)(k % NBUF);
             if (half == 0) {
                 cp_async16(&wm.pm[b][cs], &s.pm[i]);
                 cp_async16(&wm.vv[b][cs], &s.vv[i]);
@@ -211,20 +210,21 @@ __device__ __forceinline__ bool p2g_pass(const DevScene &s, P2gWarp<D, NBUF> &wm
         }
         cp_async_commit();
     };
-    auto index = [&](uint32_t k) { return k < cnt ? (src != NONE ? src + lo + k : s.perm[first + lo + k]) : 0u; };
+    auto index = [&](uint32_t k) { return k < cnt ? (src != NONE ? src + lo + k : perm[lo + k]) : 0u; };
 #pragma unroll
-    for (uint32_t k = 0; k + 1 < (uint32_t)NBUF; ++k) stage(k, index(k));
+    for (uint32_t k = 0; k + 1 < (uint32_t)NBUF; ++k) stage(k, (int)k, index(k));
     uint32_t i_next = index(NBUF - 1u);  // loaded one iteration before its copies
+    int b = 0, fill = NBUF - 1;
     for (uint32_t k = 0; k < kmax; ++k) {
-        stage(k + NBUF - 1u, i_next);
+        stage(k + NBUF - 1u, fill, i_next);
+        fill = b;
         i_next = index(k + NBUF);
         cp_async_wait<NBUF - 1>();
         __syncwarp();  // both lanes' copies of particle k have landed
         if (k < cnt) {
-            const int b = (int)(k % NBUF);
             float fdt[3] = {0.f, 0.f, 0.f};
             if constexpr (FORCE) {
-                const uint32_t i = src != NONE ? src + lo + k : s.perm[first + lo + k];
+                const uint32_t i = src != NONE ? src + lo + k : perm[lo + k];
 #pragma unroll
                 for (int d = 0; d < D; ++d) fdt[d] = s.fdt[d * n + i];
             }
@@ -234,7 +234,8 @@ __device__ __forceinline__ bool p2g_pass(const DevScene &s, P2gWarp<D, NBUF> &wm
             if (!p2g_particle<D>(wm.pm[b][cs], wm.vv[b][cs], cv, fdt, assoc, h, inv_h, half, acc))
                 atomicOr(s.err, ERR_KEY_RANGE);
         }
-        __syncwarp();  // slot k % NBUF is refilled by the next iteration's copies
+        b = b + 1 == NBUF ? 0 : b + 1;
+        __syncwarp();  // the buffer just read is refilled by the next iteration's copies
     }
     cp_async_wait<0>();
     __syncwarp();
@@ -286,17 +287,18 @@ __device__ __forceinline__ void p2g_warp_block(const DevScene &s, P2gWarp<D, NBU
     p2g_zero_tile<D>(wm);
     uint2 ord = s.bord[(size_t)r * CELLS + (lane_id() >> 1)];
     for (uint32_t pass = 0; pass < P2G_PASSES; ++pass)
-        if (!p2g_pass<D, FORCE>(s, wm, r, k.first, k.src, k.bv, k.h, k.inv_h, pass, ord, pass + 1u < P2G_PASSES)) break;
+        if (!p2g_pass<D, FORCE>(s, wm, r, s.perm + k.first, k.src, k.bv, k.h, k.inv_h, pass, ord, pass + 1u < P2G_PASSES)) break;
     __syncwarp();
     for (int t = (int)lane_id(); t < Geo<D>::TILE; t += 32) s.partial[(size_t)r * Geo<D>::TILE + t] = wm.tile[t];
     __syncwarp();
 }
 
 // Block r by a group of P2G_WARPS warps, a pass each; thread `t` of the
-// group, which `sync` synchronises.
+// group, which `sync` synchronises.  `perm`: the block's part of the
+// permutation where the group holds it, else null.
 template <int D, bool FORCE, int NBUF, typename Sync>
 __device__ __forceinline__ void p2g_group_block(const DevScene &s, P2gSmem<D, NBUF> &sm, uint32_t r, uint32_t t,
-                                                Sync sync) {
+                                                const uint32_t *perm, Sync sync) {
     constexpr int TILE = Geo<D>::TILE;
     static_assert(P2G_WARPS == P2G_PASSES, "a pass a warp");
     const uint32_t wl = t >> 5;
@@ -304,7 +306,7 @@ __device__ __forceinline__ void p2g_group_block(const DevScene &s, P2gSmem<D, NB
     if (!k.load(s, r, t == 0)) return;  // the same for the whole group
     p2g_zero_tile<D>(sm.w[wl]);
     uint2 ord = s.bord[(size_t)r * CELLS + 16u * wl + (lane_id() >> 1)];
-    p2g_pass<D, FORCE>(s, sm.w[wl], r, k.first, k.src, k.bv, k.h, k.inv_h, wl, ord, false);
+    p2g_pass<D, FORCE>(s, sm.w[wl], r, perm ? perm : s.perm + k.first, k.src, k.bv, k.h, k.inv_h, wl, ord, false);
     sync();
     for (int q = (int)t; q < TILE; q += 32 * P2G_WARPS) {
         float4 sum = sm.w[0].tile[q];
@@ -338,7 +340,7 @@ __device__ __forceinline__ void p2g_body(const DevScene &s, P2gSmem<D, NBUF> &sm
             __syncthreads();
             const uint32_t r = coop_r;
             if (r >= nb) return;
-            p2g_group_block<D, FORCE>(s, sm, r, threadIdx.x, [] { __syncthreads(); });
+            p2g_group_block<D, FORCE>(s, sm, r, threadIdx.x, nullptr, [] { __syncthreads(); });
         }
     }
     for (;;) {
@@ -441,13 +443,22 @@ template <int D> __global__ void __launch_bounds__(P2G_ATOMIC_THREADS, 4) k_p2g_
 // Colliders: Sim3/Sim2 poses, ball and cuboid projections, collide() and the
 // boundary-condition projection.
 // ---------------------------------------------------------------------------
+//
+// A sum of two products could be contracted to an FMA on either one, and a
+// product with several uses contracted or not; the compiler's choice may differ
+// between the kernels a function is inlined in.  products_sum, products_diff
+// and explicit roundings fix it, so that a stage gives the same bits in its
+// own kernel and inside k_scene_steps.
+__device__ __forceinline__ float products_diff(float a, float b, float c, float d) { return fmaf(a, b, -(c * d)); }
+__device__ __forceinline__ float products_sum(float a, float b, float c, float d) { return fmaf(a, b, c * d); }
+
 __device__ __forceinline__ void quat_rotate(const float *q, const float *v, float *out) {
-    const float t0 = 2.f * (q[1] * v[2] - q[2] * v[1]);
-    const float t1 = 2.f * (q[2] * v[0] - q[0] * v[2]);
-    const float t2 = 2.f * (q[0] * v[1] - q[1] * v[0]);
-    out[0] = v[0] + q[3] * t0 + (q[1] * t2 - q[2] * t1);
-    out[1] = v[1] + q[3] * t1 + (q[2] * t0 - q[0] * t2);
-    out[2] = v[2] + q[3] * t2 + (q[0] * t1 - q[1] * t0);
+    const float t0 = 2.f * products_diff(q[1], v[2], q[2], v[1]);
+    const float t1 = 2.f * products_diff(q[2], v[0], q[0], v[2]);
+    const float t2 = 2.f * products_diff(q[0], v[1], q[1], v[0]);
+    out[0] = fmaf(q[3], t0, v[0]) + products_diff(q[1], t2, q[2], t1);
+    out[1] = fmaf(q[3], t1, v[1]) + products_diff(q[2], t0, q[0], t2);
+    out[2] = fmaf(q[3], t2, v[2]) + products_diff(q[0], t1, q[1], t0);
 }
 
 template <int D> __device__ __forceinline__ void pose_mul_pt(const DevBody &b, const float *p, float *out) {
@@ -458,8 +469,8 @@ template <int D> __device__ __forceinline__ void pose_mul_pt(const DevBody &b, c
         for (int i = 0; i < 3; ++i) out[i] = r[i] + b.tra[i];
     } else {
         const float sp0 = p[0] * b.scale, sp1 = p[1] * b.scale;
-        out[0] = b.rot[0] * sp0 - b.rot[1] * sp1 + b.tra[0];
-        out[1] = b.rot[1] * sp0 + b.rot[0] * sp1 + b.tra[1];
+        out[0] = products_diff(b.rot[0], sp0, b.rot[1], sp1) + b.tra[0];
+        out[1] = products_sum(b.rot[1], sp0, b.rot[0], sp1) + b.tra[1];
     }
 }
 
@@ -472,8 +483,8 @@ template <int D> __device__ __forceinline__ void pose_inv_mul_pt(const DevBody &
         for (int i = 0; i < 3; ++i) out[i] = r[i] / b.scale;
     } else {
         const float d0 = p[0] - b.tra[0], d1 = p[1] - b.tra[1];
-        out[0] = (b.rot[0] * d0 + b.rot[1] * d1) / b.scale;
-        out[1] = (-b.rot[1] * d0 + b.rot[0] * d1) / b.scale;
+        out[0] = products_sum(b.rot[0], d0, b.rot[1], d1) / b.scale;
+        out[1] = products_diff(b.rot[0], d1, b.rot[1], d0) / b.scale;
     }
 }
 
@@ -801,7 +812,7 @@ template <int D, bool B = false> __device__ __forceinline__ void grid_update_bod
         }
         float cell_pos[D];
 #pragma unroll
-        for (int k = 0; k < D; ++k) cell_pos[k] = (float)(bv[k] * BW + lc[k]) * h;
+        for (int k = 0; k < D; ++k) cell_pos[k] = __fmul_rn((float)(bv[k] * BW + lc[k]), h);
         float4 nv;
         if (s.use_partial) {
             // Node sums of the deterministic P2G: the tiles of this block and
@@ -874,9 +885,9 @@ template <int D, bool B = false> __device__ __forceinline__ void grid_update_bod
 #pragma unroll
                 for (int k = 0; k < D; ++k) r[k] = cell_pos[k] - com[k];
                 if constexpr (D == 3) {
-                    vb[0] = bd.linvel[0] + bd.angvel[1] * r[2] - bd.angvel[2] * r[1];
-                    vb[1] = bd.linvel[1] + bd.angvel[2] * r[0] - bd.angvel[0] * r[2];
-                    vb[2] = bd.linvel[2] + bd.angvel[0] * r[1] - bd.angvel[1] * r[0];
+                    vb[0] = fmaf(-bd.angvel[2], r[1], fmaf(bd.angvel[1], r[2], bd.linvel[0]));
+                    vb[1] = fmaf(-bd.angvel[0], r[2], fmaf(bd.angvel[2], r[0], bd.linvel[1]));
+                    vb[2] = fmaf(-bd.angvel[1], r[0], fmaf(bd.angvel[0], r[1], bd.linvel[2]));
                 } else {
                     vb[0] = bd.linvel[0] - bd.angvel[0] * r[1];
                     vb[1] = bd.linvel[1] + bd.angvel[0] * r[0];
@@ -896,12 +907,12 @@ template <int D, bool B = false> __device__ __forceinline__ void grid_update_bod
                     float A[3];
                     int na;
                     if constexpr (D == 3) {
-                        A[0] = r[1] * J[2] - r[2] * J[1];
-                        A[1] = r[2] * J[0] - r[0] * J[2];
-                        A[2] = r[0] * J[1] - r[1] * J[0];
+                        A[0] = products_diff(r[1], J[2], r[2], J[1]);
+                        A[1] = products_diff(r[2], J[0], r[0], J[2]);
+                        A[2] = products_diff(r[0], J[1], r[1], J[0]);
                         na = 3;
                     } else {
-                        A[0] = r[0] * J[1] - r[1] * J[0];
+                        A[0] = products_diff(r[0], J[1], r[1], J[0]);
                         na = 1;
                     }
                     unsigned long long *acc = s.body_imp + (size_t)(&bd - s.bodies) * 6u;
@@ -928,7 +939,10 @@ template <int D, bool B = false> __global__ void __launch_bounds__(256, 8) k_gri
 // block counts (their readers in this substep have all run), thread g0 of
 // gs.  Done by the fused G2P / particle update, or by k_clear_next when a
 // stage hook replaced it.
-template <bool B> __device__ __forceinline__ void clear_next_map(const DevScene &s, uint32_t g0, uint32_t gs) {
+// hist: also the key histogram (a build that did not count in it leaves it
+// clear).
+template <bool B>
+__device__ __forceinline__ void clear_next_map(const DevScene &s, uint32_t g0, uint32_t gs, bool hist = true) {
     for (uint32_t q = g0; q < s.hcap; q += gs) {
         if constexpr (B) s.clr_hkeys64[q] = NONE64;
         else s.clr_hkeys[q] = NONE;
@@ -936,12 +950,15 @@ template <bool B> __device__ __forceinline__ void clear_next_map(const DevScene 
     }
     if constexpr (B) {
         for (uint32_t q = g0; q < s.n_scenes; q += gs) s.scene_nblk[q] = 0u;
-    } else {
+    } else if (hist) {
         for (uint32_t q = g0; q < HIST_BINS; q += gs) s.hist[q] = 0u;
         if (g0 < HIST_COARSE) s.hist_coarse[g0] = 0u;
     }
-    if (*s.err != 0u)
+    if (*s.err != 0u) {
         for (size_t q = g0; q < (size_t)s.hcap * CELLS; q += gs) s.slot_counts[q] = 0u;
+        if (!B && s.slot_total)
+            for (uint32_t q = g0; q < s.hcap; q += gs) s.slot_total[q] = 0u;
+    }
 }
 
 // After a stage hook replaced the fused G2P / particle update: the next
@@ -1034,8 +1051,11 @@ template <int D, int NT> struct G2pSmem {
     uint32_t next_r;
 };
 
-template <int D, int NT, bool B = false, bool POW2 = false, int MODEL = -1>
-__device__ __forceinline__ void g2p_update_body(const DevScene &s, Cta g, G2pSmem<D, NT> &sm) {
+// Particles e0, e0 + stride, ... (a thread's own) of block r, by a group of NT
+// threads (`tid` the thread in it) that `sync` synchronises.
+template <int D, int NT, bool B, bool POW2, int MODEL, typename Sync>
+__device__ __forceinline__ void g2p_block(const DevScene &s, G2pSmem<D, NT> &sm, uint32_t r, uint32_t np, uint32_t tid,
+                                          uint32_t e0, uint32_t stride, Sync sync) {
     constexpr int TW = Geo<D>::TW, TILE = Geo<D>::TILE, BW = Geo<D>::BW;
     constexpr int Q = MQ<D>::Q;
     auto &tv = sm.tv;
@@ -1043,18 +1063,11 @@ __device__ __forceinline__ void g2p_update_body(const DevScene &s, Cta g, G2pSme
     auto &st_fq = sm.st_fq;
     auto &st_fo = sm.st_fo;
     auto &st_ps = sm.st_ps;
-    const uint32_t nb = s.ctr->n_blocks;
-    float h = s.h, dt = s.dt, inv_h = s.inv_h;
-    uint32_t h_pow2 = s.h_pow2;
-    float inv_d = 4.0f / (h * h);
-    float vmax = h / dt;
     const size_t n = s.n;
-    const uint32_t tid = threadIdx.x;
-    if (s.clear_tail) clear_next_map<B>(s, g.id * NT + tid, g.n * NT);
     // Issues the copies of sorted entry e (storage index i) of the block into
     // buffer b (an empty group when e is past the block's particles).  The
     // storage index is loaded one iteration before the copies that need it.
-    auto stage = [&](int b, uint32_t e, uint32_t np, uint32_t i) {
+    auto stage = [&](int b, uint32_t e, uint32_t i) {
         if (e < np) {
             cp_async16(&st_pm[b][tid], &s.pm[i]);
 #pragma unroll
@@ -1064,10 +1077,295 @@ __device__ __forceinline__ void g2p_update_body(const DevScene &s, Cta g, G2pSme
         }
         cp_async_commit();
     };
+    const uint32_t first = s.bfirst[r];
+    // storage index of entry e: from the block's storage start when its
+    // particles are one shifted range of storage, else the permutation
+    const uint32_t src = (!B && s.reuse && s.bsrc != nullptr) ? s.bsrc[r] : NONE;
+    auto pidx = [&](uint32_t e) { return src != NONE ? src + e : s.perm[first + e]; };
+    stage(0, e0, e0 < np ? pidx(e0) : 0u);
+    uint32_t i_next = e0 + stride < np ? pidx(e0 + stride) : 0u;
+    float h = s.h, dt = s.dt, inv_h = s.inv_h;
+    uint32_t h_pow2 = s.h_pow2;
+    if constexpr (B) {
+        const SceneRec &rec = s.scenes[s.bscene[r]];
+        h = rec.h;
+        dt = rec.dt;
+        inv_h = rec.inv_h;
+        h_pow2 = rec.h_pow2;
+    }
+    const float inv_d = 4.0f / (h * h), vmax = h / dt;
+    for (uint32_t t = tid; t < TILE; t += NT) {
+        uint32_t rank, local;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tile_node_owner<D>(s, r, (int)t, rank, local)) v = s.nodes[(size_t)rank * 64u + local];
+        tv[t] = v;
+    }
+    sync();
+    int bv[D];
+    unpack_key<D>(s.bkey[r], bv);
+    int buf = 0;
+    for (uint32_t e = e0; e < np; e += stride, buf ^= 1) {
+        stage(buf ^ 1, e + stride, i_next);
+        i_next = e + 2 * stride < np ? pidx(e + 2 * stride) : 0u;
+        cp_async_wait<1>();
+        const float4 p = st_pm[buf][tid];
+        const float x[3] = {p.x, p.y, p.z};
+        float m = p.w;
+        const uint4 fo = st_fo[buf][tid];
+        uint32_t fl = fo.x;
+        // ---- G2P ----
+        float vel[D], grad[D][D], div = 0.f;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            vel[k] = 0.f;
+#pragma unroll
+            for (int l = 0; l < D; ++l) grad[k][l] = 0.f;
+        }
+        if (fl & FLAG_ENABLED) {
+            float d0[D], w[D][3];
+            int a[D];
+            bool in_block = true;
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                const float assoc = rintf(POW2 ? x[k] * inv_h : div_h(x[k], h, inv_h, h_pow2)) - 1.0f;
+                a[k] = (int)assoc - bv[k] * BW;
+                in_block = in_block && a[k] >= 0 && a[k] < BW;
+                d0[k] = fmaf(assoc, h, -x[k]);
+                bspline_weights(POW2 ? -d0[k] * inv_h : div_h(-d0[k], h, inv_h, h_pow2), w[k]);
+            }
+            if (!in_block) {  // packed-key aliasing: gather nothing
+                atomicOr(s.err, ERR_KEY_RANGE);
+#pragma unroll
+                for (int k = 0; k < D; ++k) a[k] = 0, w[k][0] = w[k][1] = w[k][2] = 0.f;
+            }
+            // Separable gather.  With w_s = wx[sx] wy[sy] wz[sz] and
+            // dpt_s = d0 + s h, the sums of g2p.slang:196-244 are
+            //   v = M0,  grad v[c][r] = inv_d (d0_r M0_c + h M_r,c),
+            //   vel_grad_det = trace(grad v),
+            // with M0 = sum_s w_s v_s and M_r = sum_s w_s s_r v_s,
+            // accumulated axis by axis.
+            // Separable gather in paired FP32 arithmetic: the node
+            // velocity (x, y, z, mass) is read as the pairs (x, y) and
+            // (z, mass); the mass lane is carried along unused.  Terms
+            // with offset 0 (s_r = 0) add nothing and are skipped.
+            constexpr int NP = (D == 3) ? 2 : 1;
+            float2 M0p[NP], Mrp[D][NP];
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                M0p[q] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < D; ++k) Mrp[k][q] = make_float2(0.f, 0.f);
+            }
+            const float2 wx0p = pair(w[0][0]), wx1p = pair(w[0][1]), wx2p = pair(w[0][2]),
+                         wx2bp = pair(2.f * w[0][2]);
+            auto row = [&](const float4 &n0, const float4 &n1, const float4 &n2, int q, float2 &R0, float2 &Rx) {
+                const float2 v0 = q ? hi_pair(n0) : lo_pair(n0), v1 = q ? hi_pair(n1) : lo_pair(n1),
+                             v2 = q ? hi_pair(n2) : lo_pair(n2);
+                R0 = __ffma2_rn(wx2p, v2, __ffma2_rn(wx1p, v1, __fmul2_rn(wx0p, v0)));
+                Rx = __ffma2_rn(wx2bp, v2, __fmul2_rn(wx1p, v1));
+            };
+            if constexpr (D == 3) {
+#pragma unroll
+                for (int sz = 0; sz < 3; ++sz) {
+                    float2 S0[2], Sx[2], Sy[2];
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) S0[q] = Sx[q] = Sy[q] = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int sy = 0; sy < 3; ++sy) {
+                        const int idx = a[0] + TW * ((a[1] + sy) + TW * (a[2] + sz));
+                        const float2 wyp = pair(w[1][sy]), wysp = pair((float)sy * w[1][sy]);
+                        const float4 n0 = tv[idx], n1 = tv[idx + 1], n2 = tv[idx + 2];
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            float2 R0, Rx;
+                            row(n0, n1, n2, q, R0, Rx);
+                            S0[q] = __ffma2_rn(wyp, R0, S0[q]);
+                            Sx[q] = __ffma2_rn(wyp, Rx, Sx[q]);
+                            if (sy > 0) Sy[q] = __ffma2_rn(wysp, R0, Sy[q]);
+                        }
+                    }
+                    const float2 wzp = pair(w[2][sz]), wzsp = pair((float)sz * w[2][sz]);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        M0p[q] = __ffma2_rn(wzp, S0[q], M0p[q]);
+                        Mrp[0][q] = __ffma2_rn(wzp, Sx[q], Mrp[0][q]);
+                        Mrp[1][q] = __ffma2_rn(wzp, Sy[q], Mrp[1][q]);
+                        if (sz > 0) Mrp[2][q] = __ffma2_rn(wzsp, S0[q], Mrp[2][q]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int sy = 0; sy < 3; ++sy) {
+                    const int idx = a[0] + TW * (a[1] + sy);
+                    const float2 wyp = pair(w[1][sy]), wysp = pair((float)sy * w[1][sy]);
+                    float2 R0, Rx;
+                    row(tv[idx], tv[idx + 1], tv[idx + 2], 0, R0, Rx);
+                    M0p[0] = __ffma2_rn(wyp, R0, M0p[0]);
+                    Mrp[0][0] = __ffma2_rn(wyp, Rx, Mrp[0][0]);
+                    if (sy > 0) Mrp[1][0] = __ffma2_rn(wysp, R0, Mrp[1][0]);
+                }
+            }
+            // v = M0, grad v[c][r] = inv_d (d0_r M0_c + h M_r,c), pairs over c
+            const float2 hp = pair(h), invdp = pair(inv_d);
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr) {
+                const float2 d0p = pair(d0[rr]);
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    const float2 g = __fmul2_rn(invdp, __ffma2_rn(d0p, M0p[q], __fmul2_rn(hp, Mrp[rr][q])));
+                    grad[2 * q][rr] = g.x;
+                    if (2 * q + 1 < D) grad[2 * q + 1][rr] = g.y;
+                }
+            }
+            vel[0] = M0p[0].x;
+            vel[1] = M0p[0].y;
+            if constexpr (D == 3) vel[2] = M0p[1].x;
+            div = grad[0][0] + grad[1][1];
+            if constexpr (D == 3) div += grad[2][2];
+        }
+        // ---- particle update ----
+        const Material &mat = s.materials[fl & FLAG_MAT_MASK];
+        const uint32_t tag = MODEL >= 0 ? (uint32_t)MODEL : mat.tag;
+        const bool fluid = tag == SLOSH_MODEL_FLUID_TAIT;
+        const bool sand = tag == SLOSH_MODEL_SAND_LINEAR || tag == SLOSH_MODEL_SAND_NEO_HOOKEAN;
+        float len2 = 0.f;
+#pragma unroll
+        for (int k = 0; k < D; ++k) len2 += vel[k] * vel[k];
+        // |v| > h / dt, tested on the squares first (sqrt is monotone; the
+        // square root is taken only for a particle near the clamp).  When
+        // (h / dt)^2 overflows, every particle takes the exact test.
+        const float vclamp2 = vmax * vmax * (1.0f - 4e-7f);
+        if (len2 > vclamp2 || isinf(vclamp2)) {
+            const float len = sqrtf(len2);
+            if (len > vmax)
+#pragma unroll
+                for (int k = 0; k < D; ++k) vel[k] = vel[k] / len * h / dt;
+        }
+        const float4 ps = (s.has_sand | s.has_damping) ? st_ps[buf][tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s.has_damping) {
+            const float dmp = 1.0f + ps.w * dt;
+#pragma unroll
+            for (int k = 0; k < D; ++k) vel[k] = vel[k] / dmp;
+        }
+        const bool fixed = (fl & FLAG_FIXED) != 0;
+        if (fixed)
+#pragma unroll
+            for (int k = 0; k < D; ++k) vel[k] = 0.f;
+        float nx[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) nx[k] = x[k] + vel[k] * dt;
+        float F[D][D];
+        {
+            float4 fv[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) fv[q] = st_fq[buf][q][tid];
+            mat_from<D>(fv, __uint_as_float(fo.w), F);
+        }
+        if (!fluid) {
+            // F <- F + (dt grad v) F, row by row in column pairs (c, c + 1)
+            float Fn[D][D];
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr) {
+                float2 g[D];
+#pragma unroll
+                for (int k = 0; k < D; ++k) g[k] = pair(grad[rr][k] * dt);
+#pragma unroll
+                for (int c = 0; c < D; c += 2) {
+                    const bool two = c + 1 < D;
+                    auto col = [&](int k) { return make_float2(F[k][c], two ? F[k][c + 1] : 0.f); };
+                    float2 acc = __fmul2_rn(col(0), g[0]);
+#pragma unroll
+                    for (int k = 1; k < D; ++k) acc = __ffma2_rn(col(k), g[k], acc);
+                    const float2 r = __fadd2_rn(make_float2(F[rr][c], two ? F[rr][c + 1] : 0.f), acc);
+                    Fn[rr][c] = r.x;
+                    if (two) Fn[rr][c + 1] = r.y;
+                }
+            }
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr)
+#pragma unroll
+                for (int c = 0; c < D; ++c) F[rr][c] = Fn[rr][c];
+        } else {
+            const float f0 = F[0][0];
+            const float nf = f0 + f0 * div * dt;
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr)
+#pragma unroll
+                for (int c = 0; c < D; ++c) F[rr][c] = (rr == c) ? nf : 0.f;
+        }
+        if (fixed)
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr)
+#pragma unroll
+                for (int c = 0; c < D; ++c) grad[rr][c] = 0.f;
+        float st[3] = {0.f, 0.f, 0.f};
+        if (sand) {
+            st[0] = ps.x;
+            st[1] = ps.y;
+            st[2] = ps.z;
+        }
+        float tau[D][D];
+        model_update<D>(mat, tag, F, st, tau, &s.ctr->n_svd_fp64);
+        const float v0 = __uint_as_float(fo.z);
+        const float coef = v0 * inv_d * dt;
+        bool finite = true;
+#pragma unroll
+        for (int k = 0; k < D; ++k) finite = finite && (nx[k] == nx[k]);
+        // The particle is stored at its canonical position o in the
+        // output buffers (contiguous, coalesced writes).
+        const size_t o = (size_t)first + e;
+        float Cn[D][D];
+        float4 np4 = p;
+        if (finite && det<D>(F) > 0.f) {
+            np4.x = nx[0];
+            np4.y = nx[1];
+            if constexpr (D == 3) np4.z = nx[2];
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr)
+#pragma unroll
+                for (int c = 0; c < D; ++c) Cn[rr][c] = products_diff(grad[rr][c], m, tau[rr][c], coef);
+        } else {
+            fl &= ~FLAG_ENABLED;
+            m = 0.f;
+            np4.w = 0.f;
+#pragma unroll
+            for (int rr = 0; rr < D; ++rr)
+#pragma unroll
+                for (int c = 0; c < D; ++c) {
+                    F[rr][c] = (rr == c) ? 1.f : 0.f;
+                    Cn[rr][c] = 0.f;
+                }
+#pragma unroll
+            for (int k = 0; k < D; ++k) vel[k] = 0.f;
+        }
+        float4 cv[Q], fv[Q];
+        const float c22 = mat_split<D>(Cn, cv), f22 = mat_split<D>(F, fv);
+        s.out_pm[o] = np4;
+        if constexpr (!B) {
+            if (s.reuse && (st_fo[buf][tid].x & FLAG_ENABLED)) note_cell_change<D, POW2>(s, r, st_pm[buf][tid], np4, h, inv_h, h_pow2);
+        }
+        s.out_vv[o] = make_float4(vel[0], vel[1], D == 3 ? vel[D - 1] : 0.f, c22);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            s.out_cq[q * n + o] = cv[q];
+            s.out_fq[q * n + o] = fv[q];
+        }
+        s.out_fo[o] = make_uint4(fl, fo.y, fo.z, __float_as_uint(f22));
+        s.out_oid[o] = fo.y;
+        if (s.has_sand | s.has_damping) s.out_ps[o] = make_float4(st[0], st[1], st[2], ps.w);
+    }
+    cp_async_wait<0>();
+}
+
+template <int D, int NT, bool B = false, bool POW2 = false, int MODEL = -1>
+__device__ __forceinline__ void g2p_update_body(const DevScene &s, Cta g, G2pSmem<D, NT> &sm) {
+    const uint32_t nb = s.ctr->n_blocks;
+    const uint32_t tid = threadIdx.x;
+    if (s.clear_tail) clear_next_map<B>(s, g.id * NT + tid, g.n * NT);
     // blocks are taken from a queue, one atomic a block
     uint32_t &next_r = sm.next_r;
     for (;;) {
-        __syncthreads();  // every thread has read next_r
+        __syncthreads();  // every thread has read next_r, and the last block's tile
         if (tid == 0) {
             if (B && s.g2p_class >= 0) {  // this launch's class of the batch's blocks
                 const uint32_t cls = (uint32_t)s.g2p_class;
@@ -1082,284 +1380,7 @@ __device__ __forceinline__ void g2p_update_body(const DevScene &s, Cta g, G2pSme
         if (r >= nb) break;
         const uint32_t np = s.bnp[r];
         if (np == 0) continue;
-        const uint32_t first = s.bfirst[r];
-        // storage index of entry e: from the block's storage start when its
-        // particles are one shifted range of storage, else the permutation
-        const uint32_t src = (!B && s.reuse && s.bsrc != nullptr) ? s.bsrc[r] : NONE;
-        auto pidx = [&](uint32_t e) { return src != NONE ? src + e : s.perm[first + e]; };
-        stage(0, tid, np, tid < np ? pidx(tid) : 0u);
-        uint32_t i_next = tid + NT < np ? pidx(tid + NT) : 0u;
-        if constexpr (B) {
-            const SceneRec &rec = s.scenes[s.bscene[r]];
-            h = rec.h;
-            dt = rec.dt;
-            inv_h = rec.inv_h;
-            h_pow2 = rec.h_pow2;
-            inv_d = 4.0f / (h * h);
-            vmax = h / dt;
-        }
-        for (int t = threadIdx.x; t < TILE; t += NT) {
-            uint32_t rank, local;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (tile_node_owner<D>(s, r, t, rank, local)) v = s.nodes[(size_t)rank * 64u + local];
-            tv[t] = v;
-        }
-        __syncthreads();
-        int bv[D];
-        unpack_key<D>(s.bkey[r], bv);
-        int buf = 0;
-        for (uint32_t e = tid; e < np; e += NT, buf ^= 1) {
-            stage(buf ^ 1, e + NT, np, i_next);
-            i_next = e + 2 * NT < np ? pidx(e + 2 * NT) : 0u;
-            cp_async_wait<1>();
-            const float4 p = st_pm[buf][tid];
-            const float x[3] = {p.x, p.y, p.z};
-            float m = p.w;
-            const uint4 fo = st_fo[buf][tid];
-            uint32_t fl = fo.x;
-            // ---- G2P ----
-            float vel[D], grad[D][D], div = 0.f;
-#pragma unroll
-            for (int k = 0; k < D; ++k) {
-                vel[k] = 0.f;
-#pragma unroll
-                for (int l = 0; l < D; ++l) grad[k][l] = 0.f;
-            }
-            if (fl & FLAG_ENABLED) {
-                float d0[D], w[D][3];
-                int a[D];
-                bool in_block = true;
-#pragma unroll
-                for (int k = 0; k < D; ++k) {
-                    const float assoc = rintf(POW2 ? x[k] * inv_h : div_h(x[k], h, inv_h, h_pow2)) - 1.0f;
-                    a[k] = (int)assoc - bv[k] * BW;
-                    in_block = in_block && a[k] >= 0 && a[k] < BW;
-                    d0[k] = assoc * h - x[k];
-                    bspline_weights(POW2 ? -d0[k] * inv_h : div_h(-d0[k], h, inv_h, h_pow2), w[k]);
-                }
-                if (!in_block) {  // packed-key aliasing: gather nothing
-                    atomicOr(s.err, ERR_KEY_RANGE);
-#pragma unroll
-                    for (int k = 0; k < D; ++k) a[k] = 0, w[k][0] = w[k][1] = w[k][2] = 0.f;
-                }
-                // Separable gather.  With w_s = wx[sx] wy[sy] wz[sz] and
-                // dpt_s = d0 + s h, the sums of g2p.slang:196-244 are
-                //   v = M0,  grad v[c][r] = inv_d (d0_r M0_c + h M_r,c),
-                //   vel_grad_det = trace(grad v),
-                // with M0 = sum_s w_s v_s and M_r = sum_s w_s s_r v_s,
-                // accumulated axis by axis.
-                // Separable gather in paired FP32 arithmetic: the node
-                // velocity (x, y, z, mass) is read as the pairs (x, y) and
-                // (z, mass); the mass lane is carried along unused.  Terms
-                // with offset 0 (s_r = 0) add nothing and are skipped.
-                constexpr int NP = (D == 3) ? 2 : 1;
-                float2 M0p[NP], Mrp[D][NP];
-#pragma unroll
-                for (int q = 0; q < NP; ++q) {
-                    M0p[q] = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int k = 0; k < D; ++k) Mrp[k][q] = make_float2(0.f, 0.f);
-                }
-                const float2 wx0p = pair(w[0][0]), wx1p = pair(w[0][1]), wx2p = pair(w[0][2]),
-                             wx2bp = pair(2.f * w[0][2]);
-                auto row = [&](const float4 &n0, const float4 &n1, const float4 &n2, int q, float2 &R0, float2 &Rx) {
-                    const float2 v0 = q ? hi_pair(n0) : lo_pair(n0), v1 = q ? hi_pair(n1) : lo_pair(n1),
-                                 v2 = q ? hi_pair(n2) : lo_pair(n2);
-                    R0 = __ffma2_rn(wx2p, v2, __ffma2_rn(wx1p, v1, __fmul2_rn(wx0p, v0)));
-                    Rx = __ffma2_rn(wx2bp, v2, __fmul2_rn(wx1p, v1));
-                };
-                if constexpr (D == 3) {
-#pragma unroll
-                    for (int sz = 0; sz < 3; ++sz) {
-                        float2 S0[2], Sx[2], Sy[2];
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) S0[q] = Sx[q] = Sy[q] = make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int sy = 0; sy < 3; ++sy) {
-                            const int idx = a[0] + TW * ((a[1] + sy) + TW * (a[2] + sz));
-                            const float2 wyp = pair(w[1][sy]), wysp = pair((float)sy * w[1][sy]);
-                            const float4 n0 = tv[idx], n1 = tv[idx + 1], n2 = tv[idx + 2];
-#pragma unroll
-                            for (int q = 0; q < 2; ++q) {
-                                float2 R0, Rx;
-                                row(n0, n1, n2, q, R0, Rx);
-                                S0[q] = __ffma2_rn(wyp, R0, S0[q]);
-                                Sx[q] = __ffma2_rn(wyp, Rx, Sx[q]);
-                                if (sy > 0) Sy[q] = __ffma2_rn(wysp, R0, Sy[q]);
-                            }
-                        }
-                        const float2 wzp = pair(w[2][sz]), wzsp = pair((float)sz * w[2][sz]);
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) {
-                            M0p[q] = __ffma2_rn(wzp, S0[q], M0p[q]);
-                            Mrp[0][q] = __ffma2_rn(wzp, Sx[q], Mrp[0][q]);
-                            Mrp[1][q] = __ffma2_rn(wzp, Sy[q], Mrp[1][q]);
-                            if (sz > 0) Mrp[2][q] = __ffma2_rn(wzsp, S0[q], Mrp[2][q]);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int sy = 0; sy < 3; ++sy) {
-                        const int idx = a[0] + TW * (a[1] + sy);
-                        const float2 wyp = pair(w[1][sy]), wysp = pair((float)sy * w[1][sy]);
-                        float2 R0, Rx;
-                        row(tv[idx], tv[idx + 1], tv[idx + 2], 0, R0, Rx);
-                        M0p[0] = __ffma2_rn(wyp, R0, M0p[0]);
-                        Mrp[0][0] = __ffma2_rn(wyp, Rx, Mrp[0][0]);
-                        if (sy > 0) Mrp[1][0] = __ffma2_rn(wysp, R0, Mrp[1][0]);
-                    }
-                }
-                // v = M0, grad v[c][r] = inv_d (d0_r M0_c + h M_r,c), pairs over c
-                const float2 hp = pair(h), invdp = pair(inv_d);
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr) {
-                    const float2 d0p = pair(d0[rr]);
-#pragma unroll
-                    for (int q = 0; q < NP; ++q) {
-                        const float2 g = __fmul2_rn(invdp, __ffma2_rn(d0p, M0p[q], __fmul2_rn(hp, Mrp[rr][q])));
-                        grad[2 * q][rr] = g.x;
-                        if (2 * q + 1 < D) grad[2 * q + 1][rr] = g.y;
-                    }
-                }
-                vel[0] = M0p[0].x;
-                vel[1] = M0p[0].y;
-                if constexpr (D == 3) vel[2] = M0p[1].x;
-                div = grad[0][0] + grad[1][1];
-                if constexpr (D == 3) div += grad[2][2];
-            }
-            // ---- particle update ----
-            const Material &mat = s.materials[fl & FLAG_MAT_MASK];
-            const uint32_t tag = MODEL >= 0 ? (uint32_t)MODEL : mat.tag;
-            const bool fluid = tag == SLOSH_MODEL_FLUID_TAIT;
-            const bool sand = tag == SLOSH_MODEL_SAND_LINEAR || tag == SLOSH_MODEL_SAND_NEO_HOOKEAN;
-            float len2 = 0.f;
-#pragma unroll
-            for (int k = 0; k < D; ++k) len2 += vel[k] * vel[k];
-            // |v| > h / dt, tested on the squares first (sqrt is monotone; the
-            // square root is taken only for a particle near the clamp).  When
-            // (h / dt)^2 overflows, every particle takes the exact test.
-            const float vclamp2 = vmax * vmax * (1.0f - 4e-7f);
-            if (len2 > vclamp2 || isinf(vclamp2)) {
-                const float len = sqrtf(len2);
-                if (len > vmax)
-#pragma unroll
-                    for (int k = 0; k < D; ++k) vel[k] = vel[k] / len * h / dt;
-            }
-            const float4 ps = (s.has_sand | s.has_damping) ? st_ps[buf][tid] : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (s.has_damping) {
-                const float dmp = 1.0f + ps.w * dt;
-#pragma unroll
-                for (int k = 0; k < D; ++k) vel[k] = vel[k] / dmp;
-            }
-            const bool fixed = (fl & FLAG_FIXED) != 0;
-            if (fixed)
-#pragma unroll
-                for (int k = 0; k < D; ++k) vel[k] = 0.f;
-            float nx[D];
-#pragma unroll
-            for (int k = 0; k < D; ++k) nx[k] = x[k] + vel[k] * dt;
-            float F[D][D];
-            {
-                float4 fv[Q];
-#pragma unroll
-                for (int q = 0; q < Q; ++q) fv[q] = st_fq[buf][q][tid];
-                mat_from<D>(fv, __uint_as_float(fo.w), F);
-            }
-            if (!fluid) {
-                // F <- F + (dt grad v) F, row by row in column pairs (c, c + 1)
-                float Fn[D][D];
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr) {
-                    float2 g[D];
-#pragma unroll
-                    for (int k = 0; k < D; ++k) g[k] = pair(grad[rr][k] * dt);
-#pragma unroll
-                    for (int c = 0; c < D; c += 2) {
-                        const bool two = c + 1 < D;
-                        auto col = [&](int k) { return make_float2(F[k][c], two ? F[k][c + 1] : 0.f); };
-                        float2 acc = __fmul2_rn(col(0), g[0]);
-#pragma unroll
-                        for (int k = 1; k < D; ++k) acc = __ffma2_rn(col(k), g[k], acc);
-                        const float2 r = __fadd2_rn(make_float2(F[rr][c], two ? F[rr][c + 1] : 0.f), acc);
-                        Fn[rr][c] = r.x;
-                        if (two) Fn[rr][c + 1] = r.y;
-                    }
-                }
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr)
-#pragma unroll
-                    for (int c = 0; c < D; ++c) F[rr][c] = Fn[rr][c];
-            } else {
-                const float f0 = F[0][0];
-                const float nf = f0 + f0 * div * dt;
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr)
-#pragma unroll
-                    for (int c = 0; c < D; ++c) F[rr][c] = (rr == c) ? nf : 0.f;
-            }
-            if (fixed)
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr)
-#pragma unroll
-                    for (int c = 0; c < D; ++c) grad[rr][c] = 0.f;
-            float st[3] = {0.f, 0.f, 0.f};
-            if (sand) {
-                st[0] = ps.x;
-                st[1] = ps.y;
-                st[2] = ps.z;
-            }
-            float tau[D][D];
-            model_update<D>(mat, tag, F, st, tau, &s.ctr->n_svd_fp64);
-            const float v0 = __uint_as_float(fo.z);
-            const float coef = v0 * inv_d * dt;
-            bool finite = true;
-#pragma unroll
-            for (int k = 0; k < D; ++k) finite = finite && (nx[k] == nx[k]);
-            // The particle is stored at its canonical position o in the
-            // output buffers (contiguous, coalesced writes).
-            const size_t o = (size_t)first + e;
-            float Cn[D][D];
-            float4 np4 = p;
-            if (finite && det<D>(F) > 0.f) {
-                np4.x = nx[0];
-                np4.y = nx[1];
-                if constexpr (D == 3) np4.z = nx[2];
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr)
-#pragma unroll
-                    for (int c = 0; c < D; ++c) Cn[rr][c] = grad[rr][c] * m - tau[rr][c] * coef;
-            } else {
-                fl &= ~FLAG_ENABLED;
-                m = 0.f;
-                np4.w = 0.f;
-#pragma unroll
-                for (int rr = 0; rr < D; ++rr)
-#pragma unroll
-                    for (int c = 0; c < D; ++c) {
-                        F[rr][c] = (rr == c) ? 1.f : 0.f;
-                        Cn[rr][c] = 0.f;
-                    }
-#pragma unroll
-                for (int k = 0; k < D; ++k) vel[k] = 0.f;
-            }
-            float4 cv[Q], fv[Q];
-            const float c22 = mat_split<D>(Cn, cv), f22 = mat_split<D>(F, fv);
-            s.out_pm[o] = np4;
-            if constexpr (!B) {
-                if (s.reuse && (st_fo[buf][tid].x & FLAG_ENABLED)) note_cell_change<D, POW2>(s, r, st_pm[buf][tid], np4, h, inv_h, h_pow2);
-            }
-            s.out_vv[o] = make_float4(vel[0], vel[1], D == 3 ? vel[D - 1] : 0.f, c22);
-#pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                s.out_cq[q * n + o] = cv[q];
-                s.out_fq[q * n + o] = fv[q];
-            }
-            s.out_fo[o] = make_uint4(fl, fo.y, fo.z, __float_as_uint(f22));
-            s.out_oid[o] = fo.y;
-            if (s.has_sand | s.has_damping) s.out_ps[o] = make_float4(st[0], st[1], st[2], ps.w);
-        }
-        cp_async_wait<0>();
-        __syncthreads();
+        g2p_block<D, NT, B, POW2, MODEL>(s, sm, r, np, tid, tid, NT, [] { __syncthreads(); });
     }
 }
 template <int D, int NT, bool B = false, bool POW2 = false, int MODEL = -1>
@@ -1378,21 +1399,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_g2p_update(DevScene s) {
 // Multi-scene batches (B): bodies of all scenes in one table, each with its
 // scene's dt and gravity (bodies of dropped scenes are left alone), and the
 // particle count in storage becomes this substep's sorted count.
-template <int D, bool B = false> __device__ __forceinline__ void rigid_body(const DevScene &s, uint32_t id) {
-    if (id == 0 && s.clear_tail) {
-        const uint32_t nb = s.ctr->n_blocks;
-        s.ctr->last_n_blocks = nb;
-        if (!build_skipped(s)) s.ctr->last_n_primary = min(s.ctr->n_primary, s.cap);
-        if (s.reuse) s.ctr->rebuild[s.par] = 0u;  // read by this substep only; G2P set the next one's
-        if constexpr (B)
-            if (s.g2p_lists)
-                for (uint32_t c = 0; c < G2P_CLASSES; ++c) s.g2p_counts[c] = 0u;  // the next block setup's lists
-        s.ctr->n_primary = 0u;
-        s.ctr->n_extra = 0u;
-        s.ctr->n_blocks = 0u;
-        if constexpr (B) *s.n_dev = nb ? s.bfirst[nb - 1] + s.bnp[nb - 1] : 0u;
-    }
-    if (id >= s.n_bodies) return;
+template <int D, bool B = false> __device__ __forceinline__ void move_body(const DevScene &s, uint32_t id) {
     DevBody b = s.bodies[id];
     float dt = s.dt, grav[3] = {s.gravity[0], s.gravity[1], s.gravity[2]};
     if constexpr (B) {
@@ -1420,7 +1427,7 @@ template <int D, bool B = false> __device__ __forceinline__ void rigid_body(cons
             float R[3][3], Iw[9];
             quat_matrix(b.rot, R);
             rotate_tensor(R, b.inv_inertia, Iw, true);
-            for (int i = 0; i < 3; ++i) b.angvel[i] += Iw[i * 3] * ja[0] + Iw[i * 3 + 1] * ja[1] + Iw[i * 3 + 2] * ja[2];
+            for (int i = 0; i < 3; ++i) b.angvel[i] += fmaf(Iw[i * 3 + 2], ja[2], products_sum(Iw[i * 3], ja[0], Iw[i * 3 + 1], ja[1]));
         } else {
             b.angvel[0] += b.inv_inertia[0] * ja[0];
         }
@@ -1441,7 +1448,7 @@ template <int D, bool B = false> __device__ __forceinline__ void rigid_body(cons
     pose_mul_pt<D>(b, b.local_com, init_com);
     if constexpr (D == 3) {
         const float sa[3] = {b.angvel[0] * dt, b.angvel[1] * dt, b.angvel[2] * dt};
-        const float ang = sqrtf(sa[0] * sa[0] + sa[1] * sa[1] + sa[2] * sa[2]);
+        const float ang = sqrtf(fmaf(sa[2], sa[2], products_sum(sa[0], sa[0], sa[1], sa[1])));
         float dq[4] = {0.f, 0.f, 0.f, 1.f};
         if (ang > 0.f) {
             const float sc = sinf(ang * 0.5f) / ang;
@@ -1453,29 +1460,45 @@ template <int D, bool B = false> __device__ __forceinline__ void rigid_body(cons
         const float rel[3] = {b.tra[0] - init_com[0], b.tra[1] - init_com[1], b.tra[2] - init_com[2]};
         float rr[3];
         quat_rotate(dq, rel, rr);
-        for (int k = 0; k < 3; ++k) b.tra[k] = init_com[k] + rr[k] * b.scale + b.linvel[k] * dt;
+        for (int k = 0; k < 3; ++k) b.tra[k] = fmaf(b.linvel[k], dt, fmaf(rr[k], b.scale, init_com[k]));
         const float *q = b.rot;
         float nq[4];
-        nq[0] = dq[3] * q[0] + dq[0] * q[3] + dq[1] * q[2] - dq[2] * q[1];
-        nq[1] = dq[3] * q[1] - dq[0] * q[2] + dq[1] * q[3] + dq[2] * q[0];
-        nq[2] = dq[3] * q[2] + dq[0] * q[1] - dq[1] * q[0] + dq[2] * q[3];
-        nq[3] = dq[3] * q[3] - dq[0] * q[0] - dq[1] * q[1] - dq[2] * q[2];
-        const float n2 = nq[0] * nq[0] + nq[1] * nq[1] + nq[2] * nq[2] + nq[3] * nq[3];
+        nq[0] = products_sum(dq[3], q[0], dq[0], q[3]) + products_diff(dq[1], q[2], dq[2], q[1]);
+        nq[1] = products_diff(dq[3], q[1], dq[0], q[2]) + products_sum(dq[1], q[3], dq[2], q[0]);
+        nq[2] = products_sum(dq[3], q[2], dq[0], q[1]) + products_diff(dq[2], q[3], dq[1], q[0]);
+        nq[3] = products_diff(dq[3], q[3], dq[0], q[0]) - products_sum(dq[1], q[1], dq[2], q[2]);
+        const float n2 = products_sum(nq[0], nq[0], nq[1], nq[1]) + products_sum(nq[2], nq[2], nq[3], nq[3]);
         const float f = 0.5f * (3.0f - n2);
         for (int k = 0; k < 4; ++k) b.rot[k] = nq[k] * f;
     } else {
         const float a = b.angvel[0] * dt;
         const float c = cosf(a), sn = sinf(a);
         const float rel0 = b.tra[0] - init_com[0], rel1 = b.tra[1] - init_com[1];
-        const float r0 = c * rel0 - sn * rel1, r1 = sn * rel0 + c * rel1;
-        b.tra[0] = init_com[0] + r0 * b.scale + b.linvel[0] * dt;
-        b.tra[1] = init_com[1] + r1 * b.scale + b.linvel[1] * dt;
-        const float nc = c * b.rot[0] - sn * b.rot[1], ns = sn * b.rot[0] + c * b.rot[1];
+        const float r0 = products_diff(c, rel0, sn, rel1), r1 = products_sum(sn, rel0, c, rel1);
+        b.tra[0] = fmaf(b.linvel[0], dt, fmaf(r0, b.scale, init_com[0]));
+        b.tra[1] = fmaf(b.linvel[1], dt, fmaf(r1, b.scale, init_com[1]));
+        const float nc = products_diff(c, b.rot[0], sn, b.rot[1]), ns = products_sum(sn, b.rot[0], c, b.rot[1]);
         b.rot[0] = nc;
         b.rot[1] = ns;
     }
     for (int k = 0; k < D; ++k) b.linvel[k] = b.linvel[k] + grav[k] * ((b.inv_mass[k] != 0.f) ? 1.f : 0.f) * dt;
     s.bodies[id] = b;
+}
+template <int D, bool B = false> __device__ __forceinline__ void rigid_body(const DevScene &s, uint32_t id) {
+    if (id == 0 && s.clear_tail) {
+        const uint32_t nb = s.ctr->n_blocks;
+        s.ctr->last_n_blocks = nb;
+        if (!build_skipped(s)) s.ctr->last_n_primary = min(s.ctr->n_primary, s.cap);
+        if (s.reuse) s.ctr->rebuild[s.par] = 0u;  // read by this substep only; G2P set the next one's
+        if constexpr (B)
+            if (s.g2p_lists)
+                for (uint32_t c = 0; c < G2P_CLASSES; ++c) s.g2p_counts[c] = 0u;  // the next block setup's lists
+        s.ctr->n_primary = 0u;
+        s.ctr->n_extra = 0u;
+        s.ctr->n_blocks = 0u;
+        if constexpr (B) *s.n_dev = nb ? s.bfirst[nb - 1] + s.bnp[nb - 1] : 0u;
+    }
+    if (id < s.n_bodies) move_body<D, B>(s, id);
 }
 template <int D, bool B = false> __global__ void k_rigid(DevScene s) {
     pdl_enter();

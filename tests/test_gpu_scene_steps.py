@@ -1,0 +1,93 @@
+"""A small scene's substeps in one cooperative launch (k_scene_steps) against
+the separate kernels (SLOSH_SCENE_STEPS=0): the same bits.
+
+The scenes sit where the one-launch form can go wrong: one particle, a block
+that does not fit its sorting buffer (768 entries), more blocks than shared
+P2G takes (16 an SM) and a count that is no multiple of 32, cell widths that
+are no power of two, two-way coupling, damping with several models, 2D; and
+more substeps than one launch holds (32), in one call and in several.
+"""
+import numpy as np
+import pytest
+
+from slosh_b200 import _lib, scenes
+from slosh_b200.pipeline import (
+    MpmData,
+    MpmPipeline,
+    ParticleModel,
+    RigidBody,
+    SimulationParams,
+    SloshError,
+    make_particles,
+)
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(pts, h, dim, model, velocities=None):
+    parts = make_particles(pts, h / 4, 1000.0, model, dim=dim, velocities=velocities)
+    floor = RigidBody(("cuboid", (4.0,) * (dim - 1) + (4.0,)), translation=(0.5,) + (-3.95,) + (0.5,) * (dim - 2),
+                      rotation=(0.0, 0.0, 0.0, 1.0) if dim == 3 else 0.0)
+    return scenes.Scene("points", dim, h, SimulationParams((0.0, -9.81, 0.0)[:dim], 1e-4), parts, [floor], 1, 1 << 15)
+
+
+def _scene(name):
+    rng = np.random.default_rng(3)
+    fluid = ParticleModel.fluid_tait(1000.0, 1.0e4, 7.0)
+    elastic = ParticleModel.elastic(1.0e5, 0.3)
+    if name == "one":
+        return _points([(0.51, 0.3, 0.47)], 1 / 64, 3, elastic, [(0.3, -1.0, 0.1)])
+    if name == "dense_block":
+        return _points(0.3 + rng.uniform(0.0, 3.9 / 64, (1000, 3)), 1 / 64, 3, elastic, rng.normal(0, 0.1, (1000, 3)))
+    if name == "scattered":
+        return _points(rng.uniform(0.1, 2.0, (2777, 3)), 1 / 64, 3, elastic, rng.normal(0, 1.0, (2777, 3)))
+    if name == "fluid_odd":
+        return _points(rng.uniform(0.1, 0.4, (4321, 2)), 1 / 50, 2, fluid, rng.normal(0, 0.5, (4321, 2)))
+    if name == "two_way":
+        return scenes.sand_column_3d(h=1 / 48, cube_coupling="two_way")
+    if name == "models":
+        sc = scenes.elastic_drop_3d(h=1 / 40)
+        other = ParticleModel.sand_neo_hookean(1.0e5, 0.3)
+        sc.particles["model_tag"][::3] = other.tag
+        sc.particles["model"][::3] = np.asarray(other.data, np.float32)
+        sc.particles["damping"][::5] = 2.0
+        sc.particles["velocity"][:, 0] = 0.3
+        return sc
+    return scenes.dam_break_2d(h=1 / 128)
+
+
+def _run(sc, monkeypatch, fused, calls):
+    monkeypatch.setenv("SLOSH_SCENE_STEPS", "1" if fused else "0")
+    data = scenes.build_mpm_data(sc)
+    pipe = MpmPipeline()
+    for n in calls:
+        pipe.launch_step(data, n)
+    out, bodies, st = data.download_particles(), data.get_bodies(), data.stats()
+    kernels = data.kernels_per_substep
+    data.close()
+    return out, bodies, st, kernels
+
+
+@pytest.mark.parametrize("name", ["one", "dense_block", "scattered", "fluid_odd", "two_way", "models", "dam"])
+def test_one_launch_matches_separate_kernels(cuda_lib, monkeypatch, name):
+    sc = _scene(name)
+    a, ab, ast, ak = _run(sc, monkeypatch, True, [1, 36])
+    b, bb, bst, bk = _run(sc, monkeypatch, False, [37])
+    assert ak == 1 and bk > 1
+    assert a.tobytes() == b.tobytes()
+    assert ab.tobytes() == bb.tobytes()
+    for k in ("n_blocks", "n_primary_blocks", "n_svd_fp64"):
+        assert ast[k] == bst[k], k
+
+
+def test_barrier_wait_is_bounded(cuda_lib, monkeypatch):
+    """The grid barrier made to wait for a CTA that never comes: the launch
+    ends by itself, the next call reports the timeout."""
+    monkeypatch.setenv("SLOSH_FUSED_BARRIER_TEST", "1:2000000")  # one arrival too many expected, 2 ms
+    sc = _scene("dam")
+    data = MpmData(sc.params, sc.particles, sc.bodies, cell_width=sc.cell_width, grid_capacity=sc.grid_capacity, dim=2)
+    MpmPipeline().launch_step(data, 3)
+    with pytest.raises(SloshError) as e:
+        data.sync()
+    assert e.value.code == _lib.SLOSH_E_TIMEOUT
+    data.close()
