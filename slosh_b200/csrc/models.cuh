@@ -124,6 +124,16 @@ __device__ __forceinline__ void neo_hookean(const float (&F)[D][D], float lambda
     for (int i = 0; i < D; ++i) tau[i][i] += diag;
 }
 
+// log(s) of a principal stretch: 2 atanh(z), z = (s - 1) / (s + 1), with
+// atanh(z) / z fitted in z^2 (Chebyshev interpolation, 3e-8 relative) for
+// stretches near 1, where s - 1 is exact.
+__device__ __forceinline__ float log_stretch(float s) {
+    const float x = s - 1.f;
+    if (!(fabsf(x) <= 0.4f)) return logf(s);
+    const float z = __fdividef(x, s + 1.f), z2 = z * z;
+    return 2.f * z * fmaf(fmaf(fmaf(1.578393363e-01f, z2, 1.993993848e-01f), z2, 3.333409452e-01f), z2, 9.999999850e-01f);
+}
+
 // Drucker-Prager projection of the singular values.  `st` = (plastic det,
 // hardening q, log_vol_gain); `p` = (h0, h1, h2, h3, lambda, mu).  On a
 // valid projection updates st, sv.s and F (= U diag(s') V^T).
@@ -137,12 +147,12 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
     const float angle = ha + (hb * q - hd) * __expf(-hc * q);
     const float s_angle = __sinf(angle);
     const float alpha = __fdividef(sqrtf(2.0f / 3.0f) * (2.0f * s_angle), 3.0f - s_angle);
-    const float d = (float)D;
+    constexpr float d = (float)D, inv_d = 1.f / (float)D;
     float strain[D], ls[D], tr = 0.f;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-        ls[i] = logf(sv.s[i]);
-        strain[i] = ls[i] + st[2] / d;
+        ls[i] = log_stretch(sv.s[i]);
+        strain[i] = fmaf(st[2], inv_d, ls[i]);
     }
 #pragma unroll
     for (int i = 0; i < D; ++i) tr += strain[i];
@@ -150,7 +160,7 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
     bool dev_zero = true;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-        dev[i] = strain[i] - tr / d;
+        dev[i] = fmaf(-tr, inv_d, strain[i]);
         dev_zero = dev_zero && (dev[i] == 0.f);
     }
     // ln of the projected singular values: log(new_det) = sum(hh) and
@@ -170,7 +180,7 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
         float n2 = 0.f;
 #pragma unroll
         for (int i = 0; i < D; ++i) n2 += dev[i] * dev[i];
-        const float devn = sqrtf(n2);
+        const float devn = n2 > 0.f ? n2 * rsqrtf(n2) : 0.f;
         const float gamma = devn + __fdividef(d * lambda + 2.0f * mu, 2.0f * mu) * tr * alpha;
         if (gamma <= 0.f) return;
         const float g = __fdividef(gamma, devn);
@@ -189,7 +199,7 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
         lprev += ls[2];
         lnew += hh[2];
     }
-    st[0] = st[0] * prev_det / new_det;
+    st[0] = __fdividef(st[0] * prev_det, new_det);
     st[2] = st[2] + lprev - lnew;
     st[1] = q + dq;
 #pragma unroll
@@ -197,21 +207,15 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
     recompose<D>(sv.U, ns, sv.V, F);
 }
 
-// The models that take principal stretches, through the SVD of F: strains
-// outside the range of stretch.cuh (rare: kept out of line, so that its
-// registers are not the particle update's).
+// Fixed-corotated stress through the SVD of F: strains outside the range of
+// stretch.cuh (rare: kept out of line, so that its registers are not the
+// particle update's).
 template <int D>
-__device__ __noinline__ void model_update_svd(const Material &mat, uint32_t tag, float (&F)[D][D], float *st,
-                                              float (&tau)[D][D], unsigned *fp64) {
+__device__ __noinline__ void corotated_svd(const float (&F)[D][D], float lambda, float mu, float (&tau)[D][D],
+                                           unsigned *fp64) {
     SvdD<D> sv;
     sv.compute(F, fp64);
-    if (tag != SLOSH_MODEL_ELASTIC_LINEAR && mat.p[7] != 0.f) drucker_prager<D>(st, mat.p + 3, sv, F);
-    if (tag == SLOSH_MODEL_SAND_NEO_HOOKEAN) {
-        neo_hookean<D>(F, mat.p[9], mat.p[10], tau);
-    } else {
-        const float *el = tag == SLOSH_MODEL_ELASTIC_LINEAR ? mat.p : mat.p + 9;
-        fixed_corotated<D>(sv, el[0], el[1], tau);
-    }
+    fixed_corotated<D>(sv, lambda, mu, tau);
 }
 
 // DefaultParticleModel::update (shaders/slosh/models/default.slang:51-92)
@@ -245,43 +249,43 @@ __device__ __forceinline__ void model_update(const Material &mat, uint32_t tag, 
                 for (int k = 0; k < D; ++k) tau[i][k] = 0.f;
             return;
     }
-    // sand without a plastic model (its lambda is 0) is purely elastic
-    const bool plastic = tag != SLOSH_MODEL_ELASTIC_LINEAR && mat.p[7] != 0.f;
-    if (tag == SLOSH_MODEL_SAND_NEO_HOOKEAN && !plastic) {
+    if (tag != SLOSH_MODEL_ELASTIC_LINEAR) {
+        // Sand keeps the SVD: its return mapping accumulates the singular
+        // values' rounding, and the stresses of sand that has barely strained
+        // are made of it, so another arithmetic gives visibly other stresses
+        // there (matrix polynomials as in stretch.cuh: C up to 9 % apart in
+        // the first substeps of a column, if closer to 64 bits; G2P of the
+        // 4.74 M-particle column 247 us instead of 307).  Without a plastic
+        // model (its lambda is 0) sand is purely elastic.
+        const bool plastic = mat.p[7] != 0.f;
+        if (tag == SLOSH_MODEL_SAND_LINEAR || plastic) {
+            SvdD<D> sv;
+            sv.compute(F, fp64);
+            if (plastic) drucker_prager<D>(st, mat.p + 3, sv, F);
+            if (tag == SLOSH_MODEL_SAND_LINEAR) {
+                fixed_corotated<D>(sv, mat.p[9], mat.p[10], tau);
+                return;
+            }
+        }
         neo_hookean<D>(F, mat.p[9], mat.p[10], tau);
         return;
     }
     Stretch<D> b;
-    bool done = b.of(F) && det<D>(F) > 0.f;
-    if (done) {
-        if (!plastic) {
-            const float *el = tag == SLOSH_MODEL_ELASTIC_LINEAR ? mat.p : mat.p + 9;
-            stretch_corotated<D>(b, el[0], el[1], tau);
-        } else if (tag == SLOSH_MODEL_SAND_LINEAR) {
-            done = stretch_sand<D, false>(b, mat.p + 3, mat.p[9], mat.p[10], st, F, tau);
-        } else {
-            done = stretch_sand<D, true>(b, mat.p + 3, mat.p[9], mat.p[10], st, F, tau);
-        }
+    if (b.of(F) && det<D>(F) > 0.f) {
+        stretch_corotated<D>(b, mat.p[0], mat.p[1], tau);
+        return;
     }
-    if (!done) {
-        // through copies, so that F, st and tau themselves stay in registers
-        float Fc[D][D], tc[D][D], sc[3] = {st[0], st[1], st[2]};
+    // through copies, so that F and tau themselves stay in registers
+    float Fc[D][D], tc[D][D];
 #pragma unroll
-        for (int i = 0; i < D; ++i)
+    for (int i = 0; i < D; ++i)
 #pragma unroll
-            for (int k = 0; k < D; ++k) Fc[i][k] = F[i][k];
-        model_update_svd<D>(mat, tag, Fc, sc, tc, fp64);
+        for (int k = 0; k < D; ++k) Fc[i][k] = F[i][k];
+    corotated_svd<D>(Fc, mat.p[0], mat.p[1], tc, fp64);
 #pragma unroll
-        for (int i = 0; i < D; ++i)
+    for (int i = 0; i < D; ++i)
 #pragma unroll
-            for (int k = 0; k < D; ++k) {
-                F[i][k] = Fc[i][k];
-                tau[i][k] = tc[i][k];
-            }
-        st[0] = sc[0];
-        st[1] = sc[1];
-        st[2] = sc[2];
-    }
+        for (int k = 0; k < D; ++k) tau[i][k] = tc[i][k];
 }
 
 }  // namespace slosh

@@ -27,7 +27,7 @@
 // 15 (every warp runs the update once, from a cold instruction cache).
 // Measured, graph of separate kernels against this, us a substep: 8,000
 // particles 50 and 38, the 62,628-particle 2D dam break 48 and 30, the
-// three-model scene of 59,049 62 and 46, the 68,921-particle sand job 62 and 52.
+// three-model scene of 59,049 62 and 48, the 68,921-particle sand job 62 and 52.
 #pragma once
 
 #include "fused.cuh"

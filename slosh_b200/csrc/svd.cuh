@@ -67,6 +67,15 @@ template <typename T> struct Svd3 {
     T offdiag;  // |R01| + |R02| + |R12| of the QR step
 };
 
+// a b + c d and a b - c d with the contraction fixed: the SVD is inlined in
+// several kernels, which must give the same bits.
+__device__ __forceinline__ float sum2(float a, float b, float c, float d) { return fmaf(a, b, c * d); }
+__device__ __forceinline__ double sum2(double a, double b, double c, double d) { return fma(a, b, c * d); }
+__device__ __forceinline__ float diff2(float a, float b, float c, float d) { return fmaf(a, b, -(c * d)); }
+__device__ __forceinline__ double diff2(double a, double b, double c, double d) { return fma(a, b, -(c * d)); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+
 // One Jacobi rotation of the symmetric matrix A (upper triangle in a[3][3])
 // in the (p, q) plane, accumulated into V.
 template <typename T, int p, int q>
@@ -77,22 +86,22 @@ __device__ __forceinline__ void jacobi_rotate(T (&a)[3][3], T (&V)[3][3]) {
     const T theta = (a[q][q] - a[p][p]) * SvdT<T>::rcp_(T(2) * apq);
     // |theta| + sqrt(theta^2 + 1) without overflow for huge theta
     const T at = fabs(theta);
-    const T den = at > T(1e15) ? T(2) * at : at + SvdT<T>::sqrt_(theta * theta + T(1));
+    const T den = at > T(1e15) ? T(2) * at : at + SvdT<T>::sqrt_(mad(theta, theta, T(1)));
     const T t = copysign(SvdT<T>::rcp_(den), theta);
-    const T c = SvdT<T>::rsqrt_(t * t + T(1));
+    const T c = SvdT<T>::rsqrt_(mad(t, t, T(1)));
     const T s = t * c;
-    a[p][p] = a[p][p] - t * apq;
-    a[q][q] = a[q][q] + t * apq;
+    a[p][p] = mad(-t, apq, a[p][p]);
+    a[q][q] = mad(t, apq, a[q][q]);
     a[p][q] = T(0);
     a[q][p] = T(0);
     const T arp = a[r][p], arq = a[r][q];
-    a[r][p] = a[p][r] = c * arp - s * arq;
-    a[r][q] = a[q][r] = s * arp + c * arq;
+    a[r][p] = a[p][r] = diff2(c, arp, s, arq);
+    a[r][q] = a[q][r] = sum2(s, arp, c, arq);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const T vp = V[i][p], vq = V[i][q];
-        V[i][p] = c * vp - s * vq;
-        V[i][q] = s * vp + c * vq;
+        V[i][p] = diff2(c, vp, s, vq);
+        V[i][q] = sum2(s, vp, c, vq);
     }
 }
 
@@ -122,21 +131,27 @@ template <typename T> __device__ __forceinline__ void givens(T a, T b, T &c, T &
     }
 }
 
-template <typename T> __device__ void svd3_impl(const T (&F)[3][3], Svd3<T> &out) {
+// The eigenvectors V of F^T F, by decreasing eigenvalue, and B = F V; `off`
+// the off-diagonal residual.  Returns whether the sweeps converged.
+template <typename T>
+__device__ __forceinline__ bool right_vectors(const T (&F)[3][3], T (&V)[3][3], T (&B)[3][3], T &off) {
     T a[3][3];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = i; j < 3; ++j) {
             T acc = F[0][i] * F[0][j];
-            acc += F[1][i] * F[1][j];
-            acc += F[2][i] * F[2][j];
+            acc = mad(F[1][i], F[1][j], acc);
+            acc = mad(F[2][i], F[2][j], acc);
             a[i][j] = acc;
             a[j][i] = acc;
         }
-    T V[3][3] = {{T(1), T(0), T(0)}, {T(0), T(1), T(0)}, {T(0), T(0), T(1)}};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) V[i][j] = T(i == j ? 1 : 0);
     bool converged = false;
-    T off = T(0);
+    off = T(0);
     for (int sweep = 0; sweep < SvdT<T>::SWEEPS; ++sweep) {
         jacobi_rotate<T, 0, 1>(a, V);
         jacobi_rotate<T, 0, 2>(a, V);
@@ -152,40 +167,48 @@ template <typename T> __device__ void svd3_impl(const T (&F)[3][3], Svd3<T> &out
     if (l0 < l1) swap_cols<T>(V, l0, l1, 0, 1);
     if (l0 < l2) swap_cols<T>(V, l0, l2, 0, 2);
     if (l1 < l2) swap_cols<T>(V, l1, l2, 1, 2);
-    // B = F V
-    T B[3][3];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) B[i][j] = F[i][0] * V[0][j] + F[i][1] * V[1][j] + F[i][2] * V[2][j];
-    if constexpr (sizeof(T) == 4) {
-        // FP32, the common case: a converged Jacobi leaves the columns of
-        // B = F V orthogonal up to its residual (B^T B = V^T F^T F V), so U is
-        // B with normalised columns.  That orthogonality error is at most
-        // the residual over s_i s_j, so this path is taken only when the
-        // singular values stay within a factor 2 of each other and F is not
-        // inverted (det B = det F); the Givens QR below keeps the other cases
-        // backward stable.
-        T n2[3];
+        for (int j = 0; j < 3; ++j) B[i][j] = mad(F[i][2], V[2][j], sum2(F[i][0], V[0][j], F[i][1], V[1][j]));
+    return converged;
+}
+
+// FP32, the common case: a converged Jacobi leaves the columns of B = F V
+// orthogonal up to its residual (B^T B = V^T F^T F V), so U is B with
+// normalised columns.  That orthogonality error is at most the residual over
+// s_i s_j, so this path is taken only when the singular values stay within a
+// factor 2 of each other and F is not inverted (det B = det F); false
+// otherwise: the Givens QR keeps the other cases backward stable.
+__device__ __forceinline__ bool normalise_columns(const float (&B)[3][3], const float (&V)[3][3], bool converged,
+                                                  Svd3<float> &out) {
+    float n2[3];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) n2[j] = B[0][j] * B[0][j] + B[1][j] * B[1][j] + B[2][j] * B[2][j];
-        const T detb = B[0][0] * (B[1][1] * B[2][2] - B[1][2] * B[2][1]) - B[0][1] * (B[1][0] * B[2][2] - B[1][2] * B[2][0]) +
-                       B[0][2] * (B[1][0] * B[2][1] - B[1][1] * B[2][0]);
-        if (converged && n2[2] > T(0.25) * n2[0] && detb > T(0)) {
+    for (int j = 0; j < 3; ++j) n2[j] = fmaf(B[2][j], B[2][j], sum2(B[0][j], B[0][j], B[1][j], B[1][j]));
+    const float c0 = diff2(B[1][1], B[2][2], B[1][2], B[2][1]), c1 = diff2(B[1][0], B[2][2], B[1][2], B[2][0]),
+                c2 = diff2(B[1][0], B[2][1], B[1][1], B[2][0]);
+    const float detb = fmaf(B[0][2], c2, diff2(B[0][0], c0, B[0][1], c1));
+    if (!(converged && n2[2] > 0.25f * n2[0] && detb > 0.f)) return false;
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const T inv = rsqrtf(n2[j]);
-                out.s[j] = n2[j] * inv;
+    for (int j = 0; j < 3; ++j) {
+        const float inv = rsqrtf(n2[j]);
+        out.s[j] = n2[j] * inv;
 #pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    out.U[i][j] = B[i][j] * inv;
-                    out.V[i][j] = V[i][j];
-                }
-            }
-            out.offdiag = off * rsqrtf(n2[0]);  // the residual, in units of s0 like R's off-diagonal
-            return;
+        for (int i = 0; i < 3; ++i) {
+            out.U[i][j] = B[i][j] * inv;
+            out.V[i][j] = V[i][j];
         }
     }
+    // a converged residual is at most 3e-7 s0^2: below the FP64 fallback's limit of 1e-5 s0 in R's units
+    out.offdiag = 0.f;
+    return true;
+}
+
+template <typename T> __device__ void svd3_impl(const T (&F)[3][3], Svd3<T> &out) {
+    T V[3][3], B[3][3], off;
+    const bool converged = right_vectors<T>(F, V, B, off);
+    if constexpr (sizeof(T) == 4)
+        if (normalise_columns(B, V, converged, out)) return;
     // QR by Givens: rows (0,1) col 0, rows (0,2) col 0, rows (1,2) col 1.
     T U[3][3] = {{T(1), T(0), T(0)}, {T(0), T(1), T(0)}, {T(0), T(0), T(1)}};
     T c, s;
@@ -283,8 +306,8 @@ template <typename T> __device__ void svd2_impl(const T (&F)[2][2], Svd2<T> &out
     const T Fm = (F[0][0] - F[1][1]) * T(0.5);
     const T G = (F[1][0] + F[0][1]) * T(0.5);
     const T H = (F[1][0] - F[0][1]) * T(0.5);
-    const T Q = sqrt(E * E + H * H);
-    const T R = sqrt(Fm * Fm + G * G);
+    const T Q = sqrt(sum2(E, E, H, H));
+    const T R = sqrt(sum2(Fm, Fm, G, G));
     const T sx = Q + R, sy = Q - R;
     const T a1 = atan2(G, Fm), a2 = atan2(H, E);
     const T theta = (a2 - a1) * T(0.5), phi = (a2 + a1) * T(0.5);

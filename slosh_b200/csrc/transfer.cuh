@@ -474,15 +474,20 @@ template <int D> __device__ __forceinline__ void pose_mul_pt(const DevBody &b, c
     }
 }
 
-template <int D> __device__ __forceinline__ void pose_inv_mul_pt(const DevBody &b, const float *p, float *out) {
+// The inverse pose of the grid node at cell * h.  Differences with a node's
+// position are formed from its cell, rounded once (here and in collide): the
+// product rounded first moves a node near a surface by a visible part of its
+// distance.
+template <int D>
+__device__ __forceinline__ void pose_inv_mul_node(const DevBody &b, const float *cell, float h, float *out) {
     if constexpr (D == 3) {
-        const float d[3] = {p[0] - b.tra[0], p[1] - b.tra[1], p[2] - b.tra[2]};
+        const float d[3] = {fmaf(cell[0], h, -b.tra[0]), fmaf(cell[1], h, -b.tra[1]), fmaf(cell[2], h, -b.tra[2])};
         const float qi[4] = {-b.rot[0], -b.rot[1], -b.rot[2], b.rot[3]};
         float r[3];
         quat_rotate(qi, d, r);
         for (int i = 0; i < 3; ++i) out[i] = r[i] / b.scale;
     } else {
-        const float d0 = p[0] - b.tra[0], d1 = p[1] - b.tra[1];
+        const float d0 = fmaf(cell[0], h, -b.tra[0]), d1 = fmaf(cell[1], h, -b.tra[1]);
         out[0] = products_sum(b.rot[0], d0, b.rot[1], d1) / b.scale;
         out[1] = products_diff(b.rot[0], d1, b.rot[1], d0) / b.scale;
     }
@@ -634,10 +639,10 @@ __device__ __forceinline__ bool cone_boundary(float hh, float r, const float *p,
 // triangle-mesh query of collide (collision/collide.slang:124-134): a mesh
 // point is returned only within `cap` of the surface.
 template <int D>
-__device__ __forceinline__ bool project_on_boundary(const DevBody &b, const float *pt, float *proj, bool &inside,
-                                                    const float4 *mvtx, const uint32_t *midx, float cap) {
+__device__ __forceinline__ bool project_on_boundary(const DevBody &b, const float *cell, float h, float *proj,
+                                                    bool &inside, const float4 *mvtx, const uint32_t *midx, float cap) {
     float local[D], lp[D];
-    pose_inv_mul_pt<D>(b, pt, local);
+    pose_inv_mul_node<D>(b, cell, h, local);
     if (b.shape_type == SLOSH_SHAPE_CUBOID) {
         float outp[D], sgn[D], diff[D], inp[D];
         bool in = true;
@@ -692,7 +697,7 @@ __device__ __forceinline__ bool project_on_boundary(const DevBody &b, const floa
 // collide (shaders/slosh/collision/collide.slang:87-153).  Returns the
 // collider id or NONE; `nd` = (normal, dot(point_node - proj, normal)).
 template <int D>
-__device__ __forceinline__ uint32_t collide(const DevBody *bodies, uint32_t n_bodies, float h, const float *pt,
+__device__ __forceinline__ uint32_t collide(const DevBody *bodies, uint32_t n_bodies, float h, const float *cell,
                                             float4 &nd, const float4 *mvtx, const uint32_t *midx) {
     const float cap = h * 1.5f;
     float best = 1.0e10f;
@@ -701,12 +706,12 @@ __device__ __forceinline__ uint32_t collide(const DevBody *bodies, uint32_t n_bo
     for (uint32_t i = 0; i < n_bodies && i < MAX_BODIES; ++i) {
         float proj[D];
         bool inside = false;
-        if (!project_on_boundary<D>(bodies[i], pt, proj, inside, mvtx, midx, cap)) continue;
+        if (!project_on_boundary<D>(bodies[i], cell, h, proj, inside, mvtx, midx, cap)) continue;
         float dpt[D], n2 = 0.f;
         bool within = true;
 #pragma unroll
         for (int k = 0; k < D; ++k) {
-            dpt[k] = proj[k] - pt[k];
+            dpt[k] = fmaf(-cell[k], h, proj[k]);
             within = within && (fabsf(dpt[k]) <= cap);
             n2 += dpt[k] * dpt[k];
         }
@@ -726,7 +731,7 @@ __device__ __forceinline__ uint32_t collide(const DevBody *bodies, uint32_t n_bo
     }
     float dd = 0.f;
 #pragma unroll
-    for (int k = 0; k < D; ++k) dd += (pt[k] - bp[k]) * bn[k];
+    for (int k = 0; k < D; ++k) dd = fmaf(fmaf(cell[k], h, -bp[k]), bn[k], dd);
     nd = make_float4(bn[0], bn[1], D == 3 ? bn[D - 1] : 0.f, dd);
     return id;
 }
@@ -810,9 +815,9 @@ template <int D, bool B = false> __device__ __forceinline__ void grid_update_bod
             lc[0] = node & 7;
             lc[1] = node >> 3;
         }
-        float cell_pos[D];
+        float cell[D];  // the node's position is cell * h
 #pragma unroll
-        for (int k = 0; k < D; ++k) cell_pos[k] = __fmul_rn((float)(bv[k] * BW + lc[k]), h);
+        for (int k = 0; k < D; ++k) cell[k] = (float)(bv[k] * BW + lc[k]);
         float4 nv;
         if (s.use_partial) {
             // Node sums of the deterministic P2G: the tiles of this block and
@@ -870,7 +875,7 @@ template <int D, bool B = false> __device__ __forceinline__ void grid_update_bod
             cid = s.prev_coll_id[(size_t)prank * 64u + node];
             if (cid != NONE) cn = s.prev_coll[(size_t)prank * 64u + node];
         } else {
-            cid = collide<D>(bodies, n_bodies, h, cell_pos, cn, s.mesh_vtx, s.mesh_idx);
+            cid = collide<D>(bodies, n_bodies, h, cell, cn, s.mesh_vtx, s.mesh_idx);
         }
         if (cid != NONE) s.coll[t] = cn;
         s.coll_id[t] = cid;
@@ -883,7 +888,7 @@ template <int D, bool B = false> __device__ __forceinline__ void grid_update_bod
                 float com[3] = {0.f, 0.f, 0.f}, r[3] = {0.f, 0.f, 0.f}, vb[3] = {0.f, 0.f, 0.f};
                 pose_mul_pt<D>(bd, bd.local_com, com);
 #pragma unroll
-                for (int k = 0; k < D; ++k) r[k] = cell_pos[k] - com[k];
+                for (int k = 0; k < D; ++k) r[k] = fmaf(cell[k], h, -com[k]);
                 if constexpr (D == 3) {
                     vb[0] = fmaf(-bd.angvel[2], r[1], fmaf(bd.angvel[1], r[2], bd.linvel[0]));
                     vb[1] = fmaf(-bd.angvel[0], r[2], fmaf(bd.angvel[2], r[0], bd.linvel[1]));

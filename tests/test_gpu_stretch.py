@@ -1,17 +1,17 @@
-"""The SVD-free constitutive update (slosh_b200/csrc/stretch.cuh) on both
+"""The SVD-free fixed-corotated stress (slosh_b200/csrc/stretch.cuh) on both
 sides of its range, against the FP64 oracle.
 
 As in test_gpu_svd.py, particles at rest carry chosen deformation gradients,
-so that one substep applies the model to F alone: F' and the plastic state are
-read back from the records, the Kirchhoff stress from C = -tau V0 (4 / h^2) dt.
+so that one substep applies the model to F alone: F' is read back from the
+records, the Kirchhoff stress from C = -tau V0 (4 / h^2) dt.
 The families put the strain at rounding size, small, moderate, just inside and
 just outside the range's edge (|X|_F = 1/2 in 3D, X^2 = I / 8 in 2D, b = F F^T
 = (1 + m)(I + X)), and well outside, under a random rotation.
 
 Tolerance.  F is FP32, so b is known to a few ulps of its entries: the stress
 carries an error of that size times the stiffness, 2e-6 (lambda + 2 mu) +
-1e-5 max |tau|, F' 1e-6 + 1e-5 max |F'| and the plastic state 1e-5 relative
-to max(1, |state|) (the bounds of test_gpu_svd.py, which cover the SVD side).
+1e-5 max |tau| and F' 1e-6 + 1e-5 max |F'| (the bounds of test_gpu_svd.py,
+which cover the SVD side).
 """
 import numpy as np
 import pytest
@@ -47,23 +47,15 @@ def _deformations(rng, dim, per):
             m = vol * rng.uniform(0.5, 1.5)
             s = np.sqrt((1.0 + m) * (1.0 + x))
             out.append(_rotation(rng, dim) @ np.diag(s) @ _rotation(rng, dim).T)
-    for _ in range(per):  # no rotation, both volume signs: Drucker-Prager's tip, shear and elastic cases
+    for _ in range(per):  # no rotation
         out.append(np.eye(dim) + 1e-3 * np.diag(rng.normal(size=dim)))
     return np.asarray(out, np.float32)
 
 
-MODELS = {
-    "fixed_corotated": ParticleModel.elastic(1.0e5, 0.3),
-    "sand": ParticleModel.sand(3.5e5, 0.3, friction_angle_deg=30.0),
-    "sand_neo_hookean": ParticleModel.sand_neo_hookean(3.0e5, 0.25),
-}
-
-
 @pytest.mark.parametrize("dim", [2, 3])
-@pytest.mark.parametrize("name", list(MODELS))
-def test_stretch_update_against_fp64_oracle(cuda_lib, name, dim):
+def test_stretch_update_against_fp64_oracle(cuda_lib, dim):
     rng = np.random.default_rng(7 + dim)
-    model = MODELS[name]
+    model = ParticleModel.elastic(1.0e5, 0.3)
     fs = _deformations(rng, dim, 40)
     n = len(fs)
     side = int(np.ceil(n ** (1 / 3)))
@@ -75,9 +67,6 @@ def test_stretch_update_against_fp64_oracle(cuda_lib, name, dim):
     for r in range(dim):
         for c in range(dim):
             recs["def_grad"][:, c * 3 + r] = fs[:, r, c]
-    sand = name != "fixed_corotated"
-    if sand:  # a pending volume correction on half of the particles
-        recs["model"][::2, 2] = -1e-3
     params = SimulationParams((0.0,) * dim, DT)
     data = MpmData(params, recs, [], cell_width=H, grid_capacity=1 << 12, dim=dim)
     MpmPipeline().launch_step(data, 1)
@@ -90,7 +79,7 @@ def test_stretch_update_against_fp64_oracle(cuda_lib, name, dim):
     ref = orc.get_particles()
 
     coef = float(recs["init_volume"][0]) * 4.0 / (H * H) * DT
-    lam, mu = (model.data[9], model.data[10]) if sand else (model.data[0], model.data[1])
+    lam, mu = model.data[0], model.data[1]
     assert np.array_equal(got["enabled"], ref["enabled"])
     tau, tau64 = got["affine"] / coef, ref["affine"] / coef
     per = n // 8
@@ -102,6 +91,3 @@ def test_stretch_update_against_fp64_oracle(cuda_lib, name, dim):
         bf = 1e-6 + 1e-5 * np.abs(ref["def_grad"][sel]).max()
         print(f"family {k}: tau err {et:.3e} (bound {bt:.3e}), F' err {ef:.3e} (bound {bf:.3e})")
         assert et <= bt and ef <= bf, k
-        if sand:
-            es = np.abs(got["model"][sel, :3] - ref["model"][sel, :3]).max(axis=0)
-            assert (es <= 1e-5 * np.maximum(1.0, np.abs(ref["model"][sel, :3]).max(axis=0))).all(), (k, es)
