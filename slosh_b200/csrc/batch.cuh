@@ -33,10 +33,12 @@ struct slosh_batch {
         bool used = false;  // holds particles in storage (live, or dropped before the next substep)
         bool live = false;
         uint32_t n = 0, body_first = 0, n_bodies = 0, tags = 0;
+        uint32_t start = 0;  // first particle of a live scene in storage
         std::vector<float> r0, phase;  // never change on the device
     };
     std::vector<Slot> slots;
     std::vector<uint32_t> dropped;  // removed since the last substep
+    bool misplaced = false;         // an error was reported: storage may have lost particles, ranges do not hold
     uint32_t n_storage = 0;         // particles in storage (mirror of *n_dev)
     uint32_t body_top = 0;          // body table entries in use
     uint32_t staging_cap = 0;       // records in c.staging
@@ -282,10 +284,25 @@ int build_batch_graphs(slosh_batch *b) {
     return SLOSH_OK;
 }
 
-int batch_check_error(slosh_batch *b) {
+// After a substep storage holds the live scenes one after another, by slot
+// (the blocks are ranked by scene): where each one starts.  The kernels that
+// read one scene read that range only; they still check every particle's scene.
+void place_scenes(slosh_batch *b) {
+    uint32_t at = 0;
+    for (auto &sl : b->slots) {
+        if (!sl.live) continue;
+        sl.start = at;
+        at += sl.n;
+    }
+}
+
+// The range of storage that holds scene `sl`: all of it after an error.
+uint32_t scene_start(const slosh_batch *b, const slosh_batch::Slot &sl) { return b->misplaced ? 0u : sl.start; }
+uint32_t scene_span(const slosh_batch *b, const slosh_batch::Slot &sl) { return b->misplaced ? b->n_storage : sl.n; }
+
+int batch_report_error(slosh_batch *b, uint32_t e) {
     slosh_ctx *c = &b->c;
-    uint32_t e = 0;
-    CK(cudaMemcpy(&e, c->err, 4, cudaMemcpyDeviceToHost));
+    b->misplaced = b->misplaced || e != 0u;
     if (e & ERR_BARRIER) {
         // the barrier words are left mid-count: restart them for the next launch
         CK(cudaMemset(&c->ctr->bar_count, 0, 2 * sizeof(uint32_t)));
@@ -296,7 +313,18 @@ int batch_check_error(slosh_batch *b) {
         CK(cudaMemset(c->err, 0, 4));
         return fail(c, SLOSH_E_CAPACITY, "a scene exceeds %u active blocks (error bits 0x%x)", SCENE_MAX_BLOCKS, e);
     }
-    return check_device_error(c);
+    return report_device_error(c, e);
+}
+int batch_check_error(slosh_batch *b) {
+    slosh_ctx *c = &b->c;
+    uint32_t e = 0;
+    CK(cudaMemcpy(&e, c->err, 4, cudaMemcpyDeviceToHost));
+    return batch_report_error(b, e);
+}
+int batch_wait_and_check(slosh_batch *b, cudaStream_t st) {
+    uint32_t e = 0;
+    if (int r = wait_and_read_error(&b->c, st, &e)) return r;
+    return batch_report_error(b, e);
 }
 
 int upload_scene_rec(slosh_batch *b, uint32_t slot, cudaStream_t st) {
@@ -626,6 +654,7 @@ int batch_activate(slosh_batch *b, cudaStream_t st) {
         CK(cudaMemcpyAsync(b->scenes_dev + sg.slot, &rec, sizeof(SceneRec), cudaMemcpyHostToDevice, st));
         slosh_batch::Slot &sl = b->slots[sg.slot];
         sl.live = true;
+        sl.start = base;
         sl.body_first = b->body_top;
         b->body_top += rec.n_bodies;
         base += sg.n;
@@ -746,6 +775,7 @@ int slosh_batch_step(slosh_batch *b, uint32_t n_substeps, void *stream) {
             b->dropped.clear();
         }
     }
+    if (n_substeps && b->n_storage) place_scenes(b);
     return SLOSH_OK;
 }
 
@@ -761,18 +791,18 @@ int slosh_batch_download_particles(slosh_batch *b, uint32_t slot, slosh_particle
         DevScene s = make_batch_scene(b, c->parity);
         IoBuffers io{};
         io.out = c->staging;
-        const uint32_t g = grid_for(b->n_storage, 256, (uint32_t)c->sm_count * 16);
-        if (c->dim == 3) k_egest<3, true><<<g, 256, 0, st>>>(s, io, slot);
-        else k_egest<2, true><<<g, 256, 0, st>>>(s, io, slot);
+        const uint32_t g = grid_for(scene_span(b, sl), 256, (uint32_t)c->sm_count * 16);
+        if (c->dim == 3) k_egest<3, true><<<g, 256, 0, st>>>(s, io, slot, scene_start(b, sl), scene_span(b, sl));
+        else k_egest<2, true><<<g, 256, 0, st>>>(s, io, slot, scene_start(b, sl), scene_span(b, sl));
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(out, c->staging, (size_t)n * sizeof(slosh_particle), cudaMemcpyDeviceToHost, st));
     }
-    CK(cudaStreamSynchronize(st));
+    const int r = batch_wait_and_check(b, st);
     for (uint32_t i = 0; i < n; ++i) {
         out[i].init_radius = sl.r0[i];
         out[i].phase = sl.phase[i];
     }
-    return batch_check_error(b);
+    return r;
 }
 
 int slosh_batch_download_positions(slosh_batch *b, uint32_t slot, float *out, uint32_t n, void *stream) {
@@ -786,12 +816,11 @@ int slosh_batch_download_positions(slosh_batch *b, uint32_t slot, float *out, ui
     if (n > 0) {
         DevScene s = make_batch_scene(b, c->parity);
         float4 *tmp = (float4 *)c->staging;  // staging holds >= 12 float4 per particle of the largest scene
-        k_positions<true><<<grid_for(b->n_storage, 256, (uint32_t)c->sm_count * 16), 256, 0, st>>>(s, tmp, slot);
+        k_positions<true><<<grid_for(scene_span(b, sl), 256, (uint32_t)c->sm_count * 16), 256, 0, st>>>(s, tmp, slot, scene_start(b, sl), scene_span(b, sl));
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(out, tmp, (size_t)n * 16, cudaMemcpyDeviceToHost, st));
     }
-    CK(cudaStreamSynchronize(st));
-    return batch_check_error(b);
+    return batch_wait_and_check(b, st);
 }
 
 int slosh_batch_get_bodies(slosh_batch *b, uint32_t slot, slosh_body *out, uint32_t n) {
@@ -816,9 +845,10 @@ int slosh_batch_timestep_bound(slosh_batch *b, uint32_t slot, float *dt_out, voi
     const DevScene s = make_batch_scene(b, c->parity);
     uint32_t *out = c->small + 3;
     CK(cudaMemsetAsync(out, 0xff, 4, st));
-    const uint32_t g = grid_for(b->n_storage, 256, (uint32_t)c->sm_count * 16);
-    if (c->dim == 3) k_timestep_bound<3, true><<<g, 256, 0, st>>>(s, slot, out);
-    else k_timestep_bound<2, true><<<g, 256, 0, st>>>(s, slot, out);
+    const slosh_batch::Slot &sl = b->slots[slot];
+    const uint32_t g = grid_for(scene_span(b, sl), 256, (uint32_t)c->sm_count * 16);
+    if (c->dim == 3) k_timestep_bound<3, true><<<g, 256, 0, st>>>(s, slot, scene_start(b, sl), scene_span(b, sl), out);
+    else k_timestep_bound<2, true><<<g, 256, 0, st>>>(s, slot, scene_start(b, sl), scene_span(b, sl), out);
     CK(cudaGetLastError());
     uint32_t u = 0;
     CK(cudaMemcpyAsync(&u, out, 4, cudaMemcpyDeviceToHost, st));
@@ -831,9 +861,10 @@ int slosh_batch_sync(slosh_batch *b, void *stream) {
     if (!b) return SLOSH_E_INVALID;
     slosh_ctx *c = &b->c;
     CK(cudaSetDevice(c->device));
-    CK(cudaStreamSynchronize(pick(c, stream)));
+    uint32_t e = 0;
+    if (int r = wait_and_read_error(c, pick(c, stream), &e)) return r;
     CK(cudaGetLastError());
-    return batch_check_error(b);
+    return batch_report_error(b, e);
 }
 
 int slosh_batch_get_stats(slosh_batch *b, slosh_batch_stats *out) {
@@ -944,6 +975,7 @@ int batch_autotune(slosh_batch *b, uint32_t substeps, void *stream, uint32_t *ra
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    place_scenes(b);
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         g_tune_cache[key] = pick_t;

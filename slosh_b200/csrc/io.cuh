@@ -155,13 +155,15 @@ __global__ void k_ingest(DevScene s, IoBuffers io, uint32_t base, uint32_t count
 }
 
 // Structure of arrays -> records, back in upload order (stored particle i is
-// record oid[i]).  Multi-scene batches (B) export the particles of one scene;
-// radius and phase are filled in by the host.
-template <int D, bool B = false> __global__ void k_egest(DevScene s, IoBuffers io, uint32_t scene) {
+// record oid[i]).  Multi-scene batches (B) export the particles of one scene,
+// which are [base, base + count) of storage; radius and phase are filled in by
+// the host.
+template <int D, bool B = false>
+__global__ void k_egest(DevScene s, IoBuffers io, uint32_t scene, uint32_t base, uint32_t count) {
     const uint32_t stride = gridDim.x * blockDim.x;
     const size_t n = s.n;
-    const uint32_t count = n_particles<B>(s);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
+    const uint32_t end = min(base + count, n_particles<B>(s));
+    for (uint32_t i = base + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += stride) {
         const uint4 fo = s.fo[i];
         if constexpr (B)
             if (scene_of(fo.x) != scene) continue;
@@ -262,16 +264,25 @@ template <int D> __global__ void k_remove_sides(DevScene s, IoBuffers io, uint32
     }
 }
 
-// Positions as vec4 (x, y, z, 0) in upload order (of one scene in B).
-template <bool B = false> __global__ void k_positions(DevScene s, float4 *out, uint32_t scene) {
+// Positions as vec4 (x, y, z, 0) in upload order of the stored particles
+// [base, base + count) (of one scene in B).  One scene reads the original
+// index from its own plane (4 bytes a particle instead of the 16 of its
+// flags), a batch the flags, which name the scene.
+template <bool B = false>
+__global__ void k_positions(DevScene s, float4 *out, uint32_t scene, uint32_t base, uint32_t count) {
     const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t count = n_particles<B>(s);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        const uint2 fo = make_uint2(s.fo[i].x, s.fo[i].y);
-        if constexpr (B)
+    const uint32_t end = min(base + count, n_particles<B>(s));
+    for (uint32_t i = base + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += stride) {
+        uint32_t id;
+        if constexpr (B) {
+            const uint4 fo = s.fo[i];
             if (scene_of(fo.x) != scene) continue;
+            id = fo.y;
+        } else {
+            id = s.oid[i];
+        }
         const float4 p = s.pm[i];
-        out[fo.y] = make_float4(p.x, p.y, p.z, 0.f);
+        out[id] = make_float4(p.x, p.y, p.z, 0.f);
     }
 }
 

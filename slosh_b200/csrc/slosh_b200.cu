@@ -9,6 +9,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <type_traits>
 #include <thread>
@@ -593,6 +595,19 @@ template <int D> bool scene_steps_fit(const slosh_ctx *c) {
     if (!ok) cudaGetLastError();
     return ok;
 }
+// The same, once for each device and dimension of the process (loading and
+// querying five kernels takes milliseconds).
+bool scene_steps_ready(const slosh_ctx *c) {
+    static std::mutex mutex;
+    static std::map<std::pair<int, int>, bool> known;
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto key = std::make_pair(c->device, c->dim);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    const bool ok = c->dim == 3 ? scene_steps_fit<3>(c) : scene_steps_fit<2>(c);
+    known[key] = ok;
+    return ok;
+}
 
 // Sets whether substeps keep their grid, from the mode and the particle
 // count; the graphs are rebuilt when that changes.
@@ -795,9 +810,8 @@ int build_graphs(slosh_ctx *c) {
     return r;
 }
 
-int check_device_error(slosh_ctx *c) {
-    uint32_t e = 0;
-    CK(cudaMemcpy(&e, c->err, 4, cudaMemcpyDeviceToHost));
+// Reports (and clears) the error bits e of work that has completed.
+int report_device_error(slosh_ctx *c, uint32_t e) {
     if (e == 0) return SLOSH_OK;
     if ((e & ERR_BARRIER) && c->slot_total) {
         // k_scene_steps left in the middle of a substep: both maps and the
@@ -821,6 +835,26 @@ int check_device_error(slosh_ctx *c) {
     if (e & (ERR_MATERIALS | ERR_MATERIAL_HASH))
         return fail(c, SLOSH_E_MATERIAL, "material table error (bits 0x%x; max %u materials)", e, MAX_MATERIALS);
     return fail(c, SLOSH_E_CUDA, "device error bits 0x%x", e);
+}
+
+int check_device_error(slosh_ctx *c) {
+    uint32_t e = 0;
+    CK(cudaMemcpy(&e, c->err, 4, cudaMemcpyDeviceToHost));
+    return report_device_error(c, e);
+}
+
+// Waits for the stream's work and reads the error bits with the same wait:
+// the end of every download (a copy of its own after the wait was a second
+// round trip of about 10 us).
+int wait_and_read_error(slosh_ctx *c, cudaStream_t st, uint32_t *e) {
+    CK(cudaMemcpyAsync(e, c->err, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return SLOSH_OK;
+}
+int wait_and_check(slosh_ctx *c, cudaStream_t st) {
+    uint32_t e = 0;
+    if (int r = wait_and_read_error(c, st, &e)) return r;
+    return report_device_error(c, e);
 }
 
 cudaStream_t pick(slosh_ctx *c, void *stream) { return stream ? (cudaStream_t)stream : c->stream; }
@@ -1007,7 +1041,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
     int coop = 0;
     c->scene_steps = c->scene_steps &&
                      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop &&
-                     (D == 3 ? scene_steps_fit<3>(c) : scene_steps_fit<2>(c));
+                     scene_steps_ready(c);
     c->reuse_mode = 2u;
     if (const char *r = std::getenv("SLOSH_GRID_REUSE")) c->reuse_mode = std::strcmp(r, "0") == 0 ? 0u : 1u;
     update_reuse(c);
@@ -1188,13 +1222,12 @@ int slosh_download_particles(slosh_ctx *c, slosh_particle *out, uint32_t n, void
         io.r0 = c->r0;
         io.phase = c->phase;
         const uint32_t g = grid_for(c->n, 256, (uint32_t)c->sm_count * 16);
-        if (c->dim == 3) k_egest<3><<<g, 256, 0, st>>>(s, io, 0u);
-        else k_egest<2><<<g, 256, 0, st>>>(s, io, 0u);
+        if (c->dim == 3) k_egest<3><<<g, 256, 0, st>>>(s, io, 0u, 0u, c->n);
+        else k_egest<2><<<g, 256, 0, st>>>(s, io, 0u, 0u, c->n);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(out, c->staging, (size_t)n * sizeof(slosh_particle), cudaMemcpyDeviceToHost, st));
     }
-    CK(cudaStreamSynchronize(st));
-    return check_device_error(c);
+    return wait_and_check(c, st);
 }
 
 int slosh_download_positions(slosh_ctx *c, float *out, uint32_t n, void *stream) {
@@ -1205,12 +1238,11 @@ int slosh_download_positions(slosh_ctx *c, float *out, uint32_t n, void *stream)
     if (n > 0) {
         DevScene s = make_scene(c, c->parity, false);
         float4 *tmp = (float4 *)c->staging;  // staging holds >= 12 float4 per particle
-        k_positions<<<grid_for(c->n, 256, (uint32_t)c->sm_count * 16), 256, 0, st>>>(s, tmp, 0u);
+        k_positions<<<grid_for(c->n, 256, (uint32_t)c->sm_count * 16), 256, 0, st>>>(s, tmp, 0u, 0u, c->n);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(out, tmp, (size_t)n * 16, cudaMemcpyDeviceToHost, st));
     }
-    CK(cudaStreamSynchronize(st));
-    return check_device_error(c);
+    return wait_and_check(c, st);
 }
 
 int slosh_set_bodies(slosh_ctx *c, const slosh_body *bodies, uint32_t n) {
@@ -1398,9 +1430,10 @@ int slosh_device_view_get(slosh_ctx *c, slosh_device_view *out) {
 int slosh_sync(slosh_ctx *c, void *stream) {
     if (!c) return SLOSH_E_INVALID;
     CK(cudaSetDevice(c->device));
-    CK(cudaStreamSynchronize(pick(c, stream)));
+    uint32_t e = 0;
+    if (int r = wait_and_read_error(c, pick(c, stream), &e)) return r;
     CK(cudaGetLastError());
-    return check_device_error(c);
+    return report_device_error(c, e);
 }
 
 uint32_t slosh_kernels_per_substep(const slosh_ctx *c) {
@@ -1619,8 +1652,8 @@ int slosh_timestep_bound(slosh_ctx *c, float *dt_out, void *stream) {
     uint32_t *slot = c->small + 3;
     CK(cudaMemsetAsync(slot, 0xff, 4, st));
     const uint32_t g = grid_for(c->n, 256, (uint32_t)c->sm_count * 16);
-    if (c->dim == 3) k_timestep_bound<3><<<g, 256, 0, st>>>(s, 0u, slot);
-    else k_timestep_bound<2><<<g, 256, 0, st>>>(s, 0u, slot);
+    if (c->dim == 3) k_timestep_bound<3><<<g, 256, 0, st>>>(s, 0u, 0u, c->n, slot);
+    else k_timestep_bound<2><<<g, 256, 0, st>>>(s, 0u, 0u, c->n, slot);
     CK(cudaGetLastError());
     uint32_t u = 0;
     CK(cudaMemcpyAsync(&u, slot, 4, cudaMemcpyDeviceToHost, st));

@@ -57,16 +57,17 @@ template <int D> __device__ __forceinline__ float det_rn(const float (&a)[D][D])
 }
 
 // One thread per stored particle; `out` holds the running minimum (reset to
-// 0xffffffff by the caller).  In batches (B) only particles of `scene`, with
-// that scene's cell width.
-template <int D, bool B = false> __global__ void k_timestep_bound(DevScene s, uint32_t scene, uint32_t *out) {
+// 0xffffffff by the caller).  In batches (B) only particles of `scene`, [base,
+// base + count) of storage, with that scene's cell width.
+template <int D, bool B = false>
+__global__ void k_timestep_bound(DevScene s, uint32_t scene, uint32_t base, uint32_t count, uint32_t *out) {
     const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t n = n_particles<B>(s);
     const size_t ps = s.n;
     uint32_t best = 0xffffffffu;
     float h = s.h;
     if constexpr (B) h = s.scenes[scene].h;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const uint32_t end = min(base + count, n_particles<B>(s));
+    for (uint32_t i = base + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += stride) {
         const uint4 fo = s.fo[i];
         const uint32_t fl = fo.x;
         if (!(fl & FLAG_ENABLED)) continue;
