@@ -147,21 +147,25 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
     const float angle = ha + (hb * q - hd) * __expf(-hc * q);
     const float s_angle = __sinf(angle);
     const float alpha = __fdividef(sqrtf(2.0f / 3.0f) * (2.0f * s_angle), 3.0f - s_angle);
-    constexpr float d = (float)D, inv_d = 1.f / (float)D;
+    const float d = (float)D;
     float strain[D], ls[D], tr = 0.f;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
         ls[i] = log_stretch(sv.s[i]);
-        strain[i] = fmaf(st[2], inv_d, ls[i]);
+        strain[i] = ls[i] + st[2] / d;
     }
 #pragma unroll
     for (int i = 0; i < D; ++i) tr += strain[i];
+    // The deviator is zero when the strains are equal: tested on the strains
+    // themselves, since strain - tr / 3 of three equal strains keeps a rounding
+    // error for one value in seven.  (Infinite strains, of a singular F, have
+    // no deviator: the particle is disabled by the NaN that follows.)
     float dev[D];
-    bool dev_zero = true;
+    bool dev_zero = fabsf(tr) < INFINITY;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-        dev[i] = fmaf(-tr, inv_d, strain[i]);
-        dev_zero = dev_zero && (dev[i] == 0.f);
+        dev[i] = strain[i] - tr / d;
+        dev_zero = dev_zero && strain[i] == strain[0];
     }
     // ln of the projected singular values: log(new_det) = sum(hh) and
     // log(prev_det) = sum(ls), so no further log is needed.

@@ -131,3 +131,36 @@ def test_svd_fp64_fallback_against_fp64_oracle(cuda_lib, model):
     must = int(((fam_of == "near_singular") | (fam_of == "inverted") | (fam_of == "isotropic")).sum())
     print(f"FP64 SVD fallbacks: {n64} (at least {must} expected)")
     assert n64 >= must
+
+
+# the three stretches equal in FP32: a multiple of a rotation that only
+# permutes and flips axes, so that F holds it without rounding
+AXIS_ROTATIONS = [
+    [[1, 0, 0], [0, 1, 0], [0, 0, 1]],
+    [[0, 1, 0], [0, 0, 1], [1, 0, 0]],
+    [[0, -1, 0], [1, 0, 0], [0, 0, 1]],
+    [[-1, 0, 0], [0, 0, 1], [0, 1, 0]],
+]
+
+
+@pytest.mark.parametrize("make", [ParticleModel.sand, ParticleModel.sand_neo_hookean], ids=["sand", "sand_neo_hookean"])
+def test_isotropic_compression_projects_to_the_tip(cuda_lib, make):
+    """Drucker-Prager's zero-deviator rule (drucker_prager.slang:150): sand
+    compressed alike along all axes loses its strain, F' = R."""
+    model = make(3.5e5, 0.3, friction_angle_deg=30.0)
+    fs = np.asarray([np.float32(c) * np.asarray(r, np.float32) for c in (0.9, 0.95, 0.99, 1.0 - 2.0**-20)
+                     for r in AXIS_ROTATIONS], np.float32)
+    recs = _scene(model, fs)
+    data = MpmData(SimulationParams((0.0, 0.0, 0.0), DT), recs, [], cell_width=H, grid_capacity=1 << 12, dim=3)
+    MpmPipeline().launch_step(data, 1)
+    got = data.download_particles()
+    data.close()
+    for i in range(len(fs)):
+        _, f64, st64 = O.model_stress(model.tag, np.asarray(model.data, np.float64), fs[i].astype(np.float64))
+        assert np.abs(f64 - np.round(f64)).max() < 1e-12, "the oracle projects to a rotation"
+        f = np.array([[got["def_grad"][i, c * 3 + r] for c in range(3)] for r in range(3)])
+        es = np.abs(got["model"][i, :3].astype(np.float64) - st64[:3])
+        print(f"F = {fs[i].tolist()}: F' err {np.abs(f - f64).max():.3e}, plastic state err {es}")
+        assert got["enabled"][i]
+        assert np.abs(f - f64).max() <= 1e-6 + 1e-5
+        assert (es <= 1e-5 * np.maximum(1.0, np.abs(st64[:3]))).all()
