@@ -124,16 +124,6 @@ __device__ __forceinline__ void neo_hookean(const float (&F)[D][D], float lambda
     for (int i = 0; i < D; ++i) tau[i][i] += diag;
 }
 
-// log(s) of a principal stretch: 2 atanh(z), z = (s - 1) / (s + 1), with
-// atanh(z) / z fitted in z^2 (Chebyshev interpolation, 3e-8 relative) for
-// stretches near 1, where s - 1 is exact.
-__device__ __forceinline__ float log_stretch(float s) {
-    const float x = s - 1.f;
-    if (!(fabsf(x) <= 0.4f)) return logf(s);
-    const float z = __fdividef(x, s + 1.f), z2 = z * z;
-    return 2.f * z * fmaf(fmaf(fmaf(1.578393363e-01f, z2, 1.993993848e-01f), z2, 3.333409452e-01f), z2, 9.999999850e-01f);
-}
-
 // Drucker-Prager projection of the singular values.  `st` = (plastic det,
 // hardening q, log_vol_gain); `p` = (h0, h1, h2, h3, lambda, mu).  On a
 // valid projection updates st, sv.s and F (= U diag(s') V^T).
@@ -151,7 +141,7 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
     float strain[D], ls[D], tr = 0.f;
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-        ls[i] = log_stretch(sv.s[i]);
+        ls[i] = logf(sv.s[i]);
         strain[i] = ls[i] + st[2] / d;
     }
 #pragma unroll
@@ -184,7 +174,7 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
         float n2 = 0.f;
 #pragma unroll
         for (int i = 0; i < D; ++i) n2 += dev[i] * dev[i];
-        const float devn = n2 > 0.f ? n2 * rsqrtf(n2) : 0.f;
+        const float devn = sqrtf(n2);
         const float gamma = devn + __fdividef(d * lambda + 2.0f * mu, 2.0f * mu) * tr * alpha;
         if (gamma <= 0.f) return;
         const float g = __fdividef(gamma, devn);
@@ -203,7 +193,7 @@ __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D
         lprev += ls[2];
         lnew += hh[2];
     }
-    st[0] = __fdividef(st[0] * prev_det, new_det);
+    st[0] = st[0] * prev_det / new_det;
     st[2] = st[2] + lprev - lnew;
     st[1] = q + dq;
 #pragma unroll

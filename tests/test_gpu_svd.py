@@ -164,3 +164,24 @@ def test_isotropic_compression_projects_to_the_tip(cuda_lib, make):
         assert got["enabled"][i]
         assert np.abs(f - f64).max() <= 1e-6 + 1e-5
         assert (es <= 1e-5 * np.maximum(1.0, np.abs(st64[:3]))).all()
+
+
+def test_log_strain_within_one_ulp(cuda_lib):
+    """The plastic state accumulates the logarithms of the principal
+    stretches.  For F = diag(s, 1, 1), s > 1 (projected to the tip), the
+    plastic determinant of one update is the singular value the kernel found
+    (times the exact stretches 1) and the log volume gain its logarithm: within
+    one ulp, the documented bound of logf."""
+    model = ParticleModel.sand(3.5e5, 0.3, friction_angle_deg=30.0)
+    ss = np.linspace(1.01, 1.6, 400)
+    fs = np.asarray([np.diag([s, 1.0, 1.0]) for s in ss], np.float32)
+    data = MpmData(SimulationParams((0.0, 0.0, 0.0), DT), _scene(model, fs), [], cell_width=H, grid_capacity=1 << 12, dim=3)
+    MpmPipeline().launch_step(data, 1)
+    got = data.download_particles()["model"]
+    data.close()
+    s = got[:, 0].astype(np.float64)
+    assert (np.abs(s - fs[:, 0, 0]) <= 2e-7 * s).all()
+    want = np.log(s)
+    ulps = np.abs(got[:, 2].astype(np.float64) - want) / np.spacing(want.astype(np.float32))
+    print(f"log of the stretch: {ulps.max():.2f} ulp")
+    assert (ulps <= 1.0).all()
