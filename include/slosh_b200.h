@@ -325,7 +325,13 @@ typedef struct slosh_device_view {
 int slosh_device_view_get(slosh_ctx *ctx, slosh_device_view *out);
 
 /* Waits for the context's work and returns the device error status
- * (SLOSH_E_OVERFLOW when the block hash map or block list overflowed). */
+ * (SLOSH_E_OVERFLOW when the block hash map or block list overflowed).
+ * SLOSH_E_TIMEOUT (here, or at a download) when a grid barrier of a small
+ * scene's one-launch substeps gave up waiting: the launch ended in the middle
+ * of a substep, so the particles hold no state any more.  Calls that read or
+ * advance them return SLOSH_E_STATE until the next slosh_upload_particles;
+ * the bodies, which moved with the substeps that completed, should be set
+ * again too. */
 int slosh_sync(slosh_ctx *ctx, void *stream);
 
 /* Number of device kernels a substep launches that runs the full grid

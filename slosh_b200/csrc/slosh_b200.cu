@@ -111,6 +111,10 @@ struct slosh_ctx {
     uint32_t *err = nullptr;
     uint32_t *small = nullptr;  // [0] n_mat, [1] scene flags, [2] debug total
     uint32_t parity = 0;
+    // A one-launch substep gave up waiting: the launch ended in mid-substep and
+    // neither buffer holds a known state.  Calls that read or advance the
+    // particles are refused until the next upload.
+    bool lost = false;
 
     slosh_particle *staging = nullptr;
 
@@ -186,7 +190,16 @@ int alloc_storage(slosh_ctx *c, slosh_ctx::Storage &S, size_t N, int D) {
         (st = dalloc(c, &S.fq, N * Q)) || (st = dalloc(c, &S.ps, N)) || (st = dalloc(c, &S.fo, N)) ||
         (st = dalloc(c, &S.oid, N)))
         return st;
+    // Zeroed, so that a buffer that a launch which gave up never wrote holds
+    // indices in range (original ids, materials) for the kernels that read it
+    // before the error does.
+    cudaMemset(S.pm, 0, N * sizeof(float4));
+    cudaMemset(S.vv, 0, N * sizeof(float4));
+    cudaMemset(S.cq, 0, N * Q * sizeof(float4));
+    cudaMemset(S.fq, 0, N * Q * sizeof(float4));
     cudaMemset(S.ps, 0, N * sizeof(float4));
+    cudaMemset(S.fo, 0, N * sizeof(uint4));
+    cudaMemset(S.oid, 0, N * 4);
     return SLOSH_OK;
 }
 
@@ -814,14 +827,19 @@ int build_graphs(slosh_ctx *c) {
 int report_device_error(slosh_ctx *c, uint32_t e) {
     if (e == 0) return SLOSH_OK;
     if ((e & ERR_BARRIER) && c->slot_total) {
-        // k_scene_steps left in the middle of a substep: both maps and the
-        // counts are cleared (while the error is set), the barrier restarts
+        // k_scene_steps left in the middle of a substep: the particles are
+        // lost; both maps, the counts (while the error is set) and the bodies'
+        // impulse sums are cleared, the barrier restarts
+        c->lost = true;
+        c->bar_extra = 0;
         for (uint32_t par = 0; par < 2; ++par)
             k_clear<false><<<(uint32_t)c->sm_count * 4, 256, 0, c->stream>>>(make_scene(c, par, false));
+        CK(cudaMemsetAsync(&c->ctr->steps_ticket, 0, 2 * sizeof(uint32_t), c->stream));
+        CK(cudaMemsetAsync(c->body_imp, 0, (size_t)MAX_BODIES * 6 * sizeof(unsigned long long), c->stream));
+        CK(cudaMemsetAsync(c->err, 0, 4, c->stream));
         CK(cudaStreamSynchronize(c->stream));
-        CK(cudaMemset(&c->ctr->steps_ticket, 0, 2 * sizeof(uint32_t)));
-        CK(cudaMemset(c->err, 0, 4));
-        return fail(c, SLOSH_E_TIMEOUT, "a grid barrier of the scene's substeps gave up waiting (error bits 0x%x)", e);
+        return fail(c, SLOSH_E_TIMEOUT,
+                    "a grid barrier of the scene's substeps gave up waiting (error bits 0x%x): upload the particles again", e);
     }
     CK(cudaMemset(c->err, 0, 4));
     if (e & (ERR_HASH_OVERFLOW | ERR_BLOCK_OVERFLOW))
@@ -855,6 +873,10 @@ int wait_and_check(slosh_ctx *c, cudaStream_t st) {
     uint32_t e = 0;
     if (int r = wait_and_read_error(c, st, &e)) return r;
     return report_device_error(c, e);
+}
+
+int refuse_lost(slosh_ctx *c) {
+    return fail(c, SLOSH_E_STATE, "the particles were lost in a substep that gave up waiting: upload them again");
 }
 
 cudaStream_t pick(slosh_ctx *c, void *stream) { return stream ? (cudaStream_t)stream : c->stream; }
@@ -1096,7 +1118,9 @@ int slosh_upload_particles(slosh_ctx *c, const slosh_particle *particles, uint32
     CK(cudaMemsetAsync(c->slot_total, 0, (size_t)c->hcap * 4, st));
     CK(cudaMemsetAsync(c->hist, 0, HIST_BINS * 4, st));
     CK(cudaMemsetAsync(c->hist_coarse, 0, HIST_COARSE * 4, st));
+    CK(cudaMemsetAsync(c->body_imp, 0, (size_t)MAX_BODIES * 6 * sizeof(unsigned long long), st));
     c->parity = 0;
+    c->lost = false;
     if (n > 0) {
         DevScene s = make_scene(c, 0, false);
         IoBuffers io{};
@@ -1131,6 +1155,7 @@ int slosh_append_particles(slosh_ctx *c, const slosh_particle *particles, uint32
     if (!c || (!particles && n)) return SLOSH_E_INVALID;
     if ((uint64_t)c->n + n > c->max_n)
         return fail(c, SLOSH_E_CAPACITY, "%u + %u particles exceed max_particles %u", c->n, n, c->max_n);
+    if (c->lost) return refuse_lost(c);
     if (n == 0) return SLOSH_OK;
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
@@ -1177,6 +1202,8 @@ int slosh_remove_particles(slosh_ctx *c, uint32_t start, uint32_t count, uint32_
     if (!c) return SLOSH_E_INVALID;
     const uint32_t end = (uint32_t)std::min<uint64_t>((uint64_t)start + count, c->n);
     const uint32_t nrem = start < end ? end - start : 0u;
+    if (removed) *removed = 0;
+    if (c->lost) return refuse_lost(c);
     if (removed) *removed = nrem;
     if (nrem == 0) return SLOSH_OK;
     CK(cudaSetDevice(c->device));
@@ -1213,6 +1240,7 @@ int slosh_remove_particles(slosh_ctx *c, uint32_t start, uint32_t count, uint32_
 int slosh_download_particles(slosh_ctx *c, slosh_particle *out, uint32_t n, void *stream) {
     if (!c || (!out && n)) return SLOSH_E_INVALID;
     if (n > c->n) return fail(c, SLOSH_E_INVALID, "asked for %u particles, context holds %u", n, c->n);
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     if (n > 0) {
@@ -1233,6 +1261,7 @@ int slosh_download_particles(slosh_ctx *c, slosh_particle *out, uint32_t n, void
 int slosh_download_positions(slosh_ctx *c, float *out, uint32_t n, void *stream) {
     if (!c || (!out && n)) return SLOSH_E_INVALID;
     if (n > c->n) return fail(c, SLOSH_E_INVALID, "asked for %u particles, context holds %u", n, c->n);
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     if (n > 0) {
@@ -1322,6 +1351,7 @@ int slosh_get_bodies(slosh_ctx *c, slosh_body *out, uint32_t n) {
 int slosh_step(slosh_ctx *c, uint32_t n_substeps, void *stream) {
     if (!c) return SLOSH_E_INVALID;
     if (c->n == 0) return fail(c, SLOSH_E_STATE, "no particles uploaded");
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     for (uint32_t k = 0; k < n_substeps; ++k) {
@@ -1451,6 +1481,7 @@ int slosh_profile_substeps(slosh_ctx *c, uint32_t n_substeps, void *stream, floa
                            uint32_t *n_kernels) {
     if (!c || (!kernel_ms && cap)) return SLOSH_E_INVALID;
     if (c->n == 0) return fail(c, SLOSH_E_STATE, "no particles uploaded");
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     Prof pr{};
     pr.st = pick(c, stream);
@@ -1515,6 +1546,7 @@ int slosh_kernel_name(uint32_t index, char *buf, size_t len) {
 int slosh_grid_debug(slosh_ctx *c, slosh_grid_dump *dump, uint32_t cap_blocks, uint32_t cap_sorted) {
     if (!c || !dump) return SLOSH_E_INVALID;
     if (c->n == 0) return fail(c, SLOSH_E_STATE, "no particles uploaded");
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
     DevScene s = make_scene(c, c->parity, false);
@@ -1599,6 +1631,7 @@ int slosh_grid_debug(slosh_ctx *c, slosh_grid_dump *dump, uint32_t cap_blocks, u
 int slosh_debug_nodes(slosh_ctx *c, int stage, float *nodes, uint32_t cap_blocks, uint32_t *n_blocks) {
     if (!c || stage < 1 || stage > 2) return SLOSH_E_INVALID;
     if (c->n == 0) return fail(c, SLOSH_E_STATE, "no particles uploaded");
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     cudaStream_t st = c->stream;
     DevScene s = make_scene(c, c->parity, c->force_pending != 0);
@@ -1646,6 +1679,7 @@ int slosh_prefix_sum(slosh_ctx *c, const uint32_t *in, uint32_t *out, uint32_t n
 int slosh_timestep_bound(slosh_ctx *c, float *dt_out, void *stream) {
     if (!c || !dt_out) return SLOSH_E_INVALID;
     if (c->n == 0) return fail(c, SLOSH_E_STATE, "no particles uploaded");
+    if (c->lost) return refuse_lost(c);
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     const DevScene s = make_scene(c, c->parity, false);
@@ -1655,9 +1689,10 @@ int slosh_timestep_bound(slosh_ctx *c, float *dt_out, void *stream) {
     if (c->dim == 3) k_timestep_bound<3><<<g, 256, 0, st>>>(s, 0u, 0u, c->n, slot);
     else k_timestep_bound<2><<<g, 256, 0, st>>>(s, 0u, 0u, c->n, slot);
     CK(cudaGetLastError());
-    uint32_t u = 0;
+    uint32_t u = 0, e = 0;
     CK(cudaMemcpyAsync(&u, slot, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    if (int r = wait_and_read_error(c, st, &e)) return r;
+    if (e & ERR_BARRIER) return report_device_error(c, e);  // the bound is of no known state
     *dt_out = (float)u / TIMESTEP_FLOAT_TO_INT;  // GpuTimestepBounds::computed_dt
     return SLOSH_OK;
 }

@@ -80,14 +80,46 @@ def test_one_launch_matches_separate_kernels(cuda_lib, monkeypatch, name):
         assert ast[k] == bst[k], k
 
 
-def test_barrier_wait_is_bounded(cuda_lib, monkeypatch):
+@pytest.mark.parametrize("reported_by", ["sync", "positions", "timestep_bound"])
+def test_barrier_wait_is_bounded(cuda_lib, monkeypatch, reported_by):
     """The grid barrier made to wait for a CTA that never comes: the launch
-    ends by itself, the next call reports the timeout."""
-    monkeypatch.setenv("SLOSH_FUSED_BARRIER_TEST", "1:2000000")  # one arrival too many expected, 2 ms
+    ends by itself, the next call reports the timeout, calls on the lost
+    particles are refused, and an upload makes the context whole again."""
     sc = _scene("dam")
-    data = MpmData(sc.params, sc.particles, sc.bodies, cell_width=sc.cell_width, grid_capacity=sc.grid_capacity, dim=2)
-    MpmPipeline().launch_step(data, 3)
+
+    def fresh():
+        return MpmData(sc.params, sc.particles, sc.bodies, cell_width=sc.cell_width, grid_capacity=sc.grid_capacity,
+                       dim=2, max_particles=sc.n + 1)
+
+    pipe = MpmPipeline()
+    want = fresh()
+    pipe.launch_step(want, 3)
+    monkeypatch.setenv("SLOSH_FUSED_BARRIER_TEST", "1:2000000")  # one arrival too many expected, 2 ms
+    data = fresh()
+    pipe.launch_step(data, 3)
     with pytest.raises(SloshError) as e:
-        data.sync()
+        getattr(data, reported_by)()
     assert e.value.code == _lib.SLOSH_E_TIMEOUT
+    refused = [
+        lambda: pipe.launch_step(data, 1),
+        data.positions,
+        data.download_particles,
+        data.timestep_bound,
+        lambda: data.append(sc.particles[:1]),
+        lambda: data.shift_remove(0, 1),
+        lambda: data.profile_substeps(1),
+        data.grid_debug,
+        lambda: data.debug_nodes(1),
+    ]
+    for call in refused:
+        with pytest.raises(SloshError) as e:
+            call()
+        assert e.value.code == _lib.SLOSH_E_STATE
+    data.upload(sc.particles)
+    data.set_bodies(sc.bodies)
+    pipe.launch_step(data, 3)
+    assert data.kernels_per_substep == 1
+    assert data.download_particles().tobytes() == want.download_particles().tobytes()
+    assert data.get_bodies().tobytes() == want.get_bodies().tobytes()
     data.close()
+    want.close()
