@@ -400,23 +400,23 @@ template <int NT> __device__ __forceinline__ uint32_t cta_scan_vec16(const uint3
     return carry;
 }
 
-// Exclusive scan of the key histogram and the final block count.  CTA c
-// scans bins [1024 c, 1024 c + 1024), one uint4 a thread, on top of the
+// Exclusive scan of the key histogram: a CTA of NT >= 256 threads scans bins
+// [1024 c, 1024 c + 1024), one uint4 a thread of the first 256, on top of the
 // coarse counts of the bins before them.
-template <int NT> __global__ void __launch_bounds__(NT) k_hist_scan(DevScene s) {
-    pdl_enter();
-    if (build_skipped(s)) return;  // this substep keeps the previous grid
-    constexpr uint32_t PER = HIST_BINS / HIST_COARSE, NW = NT / 32;
-    static_assert(PER == 4 * NT && HIST_COARSE <= 64, "one uint4 of bins a thread");
+template <int NT> __device__ __forceinline__ void hist_scan_part(const DevScene &s, uint32_t c) {
+    constexpr uint32_t PER = HIST_BINS / HIST_COARSE, VECS = PER / 4, NW = VECS / 32;
+    static_assert(NT >= (int)VECS && HIST_COARSE <= 64, "one uint4 of bins a thread");
     __shared__ uint32_t wtot[NW];
     __shared__ uint32_t base;
-    const uint32_t lane = lane_id(), w = threadIdx.x >> 5, c = blockIdx.x;
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const bool mine = threadIdx.x < VECS;
     if (w == 0) {
         uint32_t v = (lane < c ? s.hist_coarse[lane] : 0u) + (lane + 32u < c ? s.hist_coarse[lane + 32u] : 0u);
         v = __reduce_add_sync(FULL_MASK, v);
         if (lane == 0) base = v;
     }
-    const uint4 v = reinterpret_cast<const uint4 *>(s.hist + (size_t)c * PER)[threadIdx.x];
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (mine) v = reinterpret_cast<const uint4 *>(s.hist + (size_t)c * PER)[threadIdx.x];
     const uint32_t sum = v.x + v.y + v.z + v.w;
     uint32_t incl = sum;
 #pragma unroll
@@ -424,17 +424,27 @@ template <int NT> __global__ void __launch_bounds__(NT) k_hist_scan(DevScene s) 
         const uint32_t y = __shfl_up_sync(FULL_MASK, incl, off);
         if (lane >= (uint32_t)off) incl += y;
     }
-    if (lane == 31) wtot[w] = incl;
+    if (mine && lane == 31) wtot[w] = incl;
     __syncthreads();
-    uint32_t pre = base;
-    for (uint32_t q = 0; q < w; ++q) pre += wtot[q];
-    uint4 o;
-    o.x = pre + incl - sum;
-    o.y = o.x + v.x;
-    o.z = o.y + v.y;
-    o.w = o.z + v.z;
-    reinterpret_cast<uint4 *>(s.hist_start + (size_t)c * PER)[threadIdx.x] = o;
-    if (c == 0 && threadIdx.x == 0) {
+    if (mine) {
+        uint32_t pre = base;
+        for (uint32_t q = 0; q < w; ++q) pre += wtot[q];
+        uint4 o;
+        o.x = pre + incl - sum;
+        o.y = o.x + v.x;
+        o.z = o.y + v.y;
+        o.w = o.z + v.z;
+        reinterpret_cast<uint4 *>(s.hist_start + (size_t)c * PER)[threadIdx.x] = o;
+    }
+    __syncthreads();  // the sums are read; the next part overwrites them
+}
+
+// The key histogram's scan, a CTA a coarse bin, and the final block count.
+template <int NT> __global__ void __launch_bounds__(NT) k_hist_scan(DevScene s) {
+    pdl_enter();
+    if (build_skipped(s)) return;  // this substep keeps the previous grid
+    hist_scan_part<NT>(s, blockIdx.x);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t total = min(s.ctr->n_primary, s.cap) + min(s.ctr->n_extra, s.cap);
         if (total > s.cap) atomicOr(s.err, ERR_BLOCK_OVERFLOW);
         s.ctr->n_blocks = min(total, s.cap);

@@ -10,7 +10,10 @@
 //             neighbours inserted                       (k_touch, k_neighbors)
 //   rank      a warp per block: its rank and first entry, as the number of
 //             smaller keys and the particles in their blocks; its cells
-//                              (k_hist_scan .. k_block_setup, k_block_scan)
+//                              (k_hist_scan .. k_block_setup, k_block_scan).
+//             Above STEPS_KEYS blocks all pairs are too many (24,000 blocks:
+//             2,970 us a substep): the separate kernels' key histogram, with
+//             four barriers more (255 us)
 //   scatter   the permutation; the blocks' neighbour ranks     (k_scatter)
 //   transfer  four warps per block: canonical order, then P2G  (k_canon, k_p2g)
 //   update    the grid nodes                              (k_grid_update)
@@ -36,7 +39,7 @@ namespace slosh {
 
 constexpr int STEPS_THREADS = 512;
 constexpr uint32_t STEPS_GROUPS = STEPS_THREADS / 128;  // groups of four warps: a P2G block, a G2P CTA
-constexpr uint32_t STEPS_KEYS = 8192;                   // block keys ranked from shared memory
+constexpr uint32_t STEPS_KEYS = 4096;                   // block keys ranked all against all, from shared memory
 
 // The scene as substeps of either parity see it.
 struct ScenePair {
@@ -173,38 +176,27 @@ template <int D> __device__ __forceinline__ void steps_touch(const DevScene &s) 
     }
 }
 
-// Ranks, first entries and cells of the listed blocks.
-template <int D> __device__ __forceinline__ void steps_rank(const DevScene &s, StepsSmem<D> &sm) {
-    const uint32_t total = min(s.ctr->n_extra, s.cap);
+// Ranks, first entries and cells of up to STEPS_KEYS listed blocks, a warp a
+// block: the smaller keys, and the particles in their blocks, counted over all
+// keys in shared memory.
+template <int D> __device__ __forceinline__ void steps_rank(const DevScene &s, StepsSmem<D> &sm, uint32_t total) {
     const uint32_t lane = lane_id();
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     if (blockIdx.x == 0 && threadIdx.x == 0) s.ctr->n_blocks = total;
-    const uint32_t w0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const bool staged = total <= STEPS_KEYS;
     if (blockIdx.x >= total) return;  // no warp of this CTA has a block
-    if (staged) {
-        for (uint32_t q = threadIdx.x; q < total; q += blockDim.x) {
-            sm.rank.key[q] = s.blist_key[q];
-            sm.rank.count[q] = s.slot_total[s.blist_slot[q]];
-        }
-        __syncthreads();
+    for (uint32_t q = threadIdx.x; q < total; q += blockDim.x) {
+        sm.rank.key[q] = s.blist_key[q];
+        sm.rank.count[q] = s.slot_total[s.blist_slot[q]];
     }
-    for (uint32_t j = w0; j < total; j += warps) {
-        const uint32_t key = s.blist_key[j], slot = s.blist_slot[j];
+    __syncthreads();
+    for (uint32_t j = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; j < total; j += warps) {
+        const uint32_t key = sm.rank.key[j], slot = s.blist_slot[j];
         uint32_t r = 0, first = 0;
-        if (staged) {
 #pragma unroll 4
-            for (uint32_t q = lane; q < total; q += 32u) {
-                const bool less = sm.rank.key[q] < key;
-                r += less ? 1u : 0u;
-                first += less ? sm.rank.count[q] : 0u;
-            }
-        } else {
-            for (uint32_t q = lane; q < total; q += 32u) {
-                const bool less = s.blist_key[q] < key;
-                r += less ? 1u : 0u;
-                first += less ? s.slot_total[s.blist_slot[q]] : 0u;
-            }
+        for (uint32_t q = lane; q < total; q += 32u) {
+            const bool less = sm.rank.key[q] < key;
+            r += less ? 1u : 0u;
+            first += less ? sm.rank.count[q] : 0u;
         }
         r = __reduce_add_sync(FULL_MASK, r);
         first = __reduce_add_sync(FULL_MASK, first);
@@ -216,6 +208,58 @@ template <int D> __device__ __forceinline__ void steps_rank(const DevScene &s, S
             s.hvals[slot] = r | (np ? 0u : RANK_EXTRA);
             if (np) atomicAdd(&s.ctr->n_primary, 1u);
         }
+    }
+}
+
+// The same for more blocks, in time linear in them: by the key histogram and
+// its bins, as the separate kernels rank (k_neighbors' counts, k_hist_scan,
+// k_bin_scatter, k_rank, k_block_scan), with four more barriers.  The histogram
+// is clear on entry; steps_clear_hist clears it once the ranks are used.
+template <int D>
+__device__ __forceinline__ bool steps_rank_many(const DevScene &s, uint32_t total, uint32_t &round, uint32_t *flag) {
+    const uint32_t lane = lane_id();
+    const uint32_t threads = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t0 == 0) s.ctr->n_blocks = total;
+    for (uint32_t base = t0 - lane; base < total; base += threads) {
+        const uint32_t t = base + lane;
+        const uint32_t key = t < total ? s.blist_key[t] : 0u, coarse = t < total ? key >> 26 : NONE;
+        if (t < total) atomicAdd(&s.hist[key >> 16], 1u);
+        const unsigned peers = __match_any_sync(FULL_MASK, coarse);
+        if (coarse != NONE && (int)lane == __ffs(peers) - 1) atomicAdd(&s.hist_coarse[coarse], (uint32_t)__popc(peers));
+    }
+    if (!steps_barrier(s, round, flag)) return false;
+    for (uint32_t c = blockIdx.x; c < HIST_COARSE; c += gridDim.x) hist_scan_part<STEPS_THREADS>(s, c);
+    if (!steps_barrier(s, round, flag)) return false;
+    for (uint32_t t = t0; t < total; t += threads) {
+        const uint32_t key = s.blist_key[t], pos = atomicAdd(&s.hist_start[key >> 16], 1u);
+        s.tmp_key[pos] = key;
+        s.tmp_slot[pos] = s.blist_slot[t];
+    }
+    if (!steps_barrier(s, round, flag)) return false;
+    for (uint32_t t = t0 >> 5; t < total; t += threads >> 5) {
+        const uint32_t key = s.tmp_key[t], slot = s.tmp_slot[t];
+        const uint32_t end = s.hist_start[key >> 16], start = end - s.hist[key >> 16];  // advanced by the scatter
+        uint32_t r = 0;
+#pragma unroll 4
+        for (uint32_t q = start + lane; q < end; q += 32u) r += s.tmp_key[q] < key ? 1u : 0u;
+        r = start + __reduce_add_sync(FULL_MASK, r);
+        const uint32_t np = block_cells(s, r, slot);
+        if (lane == 0) {
+            s.bkey[r] = key;
+            s.bslot[r] = slot;
+            s.hvals[slot] = r | (np ? 0u : RANK_EXTRA);
+            if (np) atomicAdd(&s.ctr->n_primary, 1u);
+        }
+    }
+    if (!steps_barrier(s, round, flag)) return false;
+    if (blockIdx.x == 0) block_scan_body<STEPS_THREADS>(s);
+    return true;
+}
+__device__ __forceinline__ void steps_clear_hist(const DevScene &s, uint32_t nb) {
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nb; r += gridDim.x * blockDim.x) {
+        const uint32_t key = s.bkey[r];
+        s.hist[key >> 16] = 0u;
+        s.hist_coarse[key >> 26] = 0u;
     }
 }
 
@@ -269,9 +313,11 @@ __global__ void __launch_bounds__(STEPS_THREADS, 1)
         if (k && !(alive = steps_barrier(s, round, &flag))) break;
         steps_touch<D>(s);
         if (!(alive = steps_barrier(s, round, &flag))) break;
-        steps_rank<D>(s, sm);
+        const uint32_t nb = min(s.ctr->n_extra, s.cap);
+        if (nb <= STEPS_KEYS) steps_rank<D>(s, sm, nb);
+        else if (!(alive = steps_rank_many<D>(s, nb, round, &flag))) break;
         if (!(alive = steps_barrier(s, round, &flag))) break;
-        const uint32_t nb = s.ctr->n_blocks;
+        if (nb > STEPS_KEYS) steps_clear_hist(s, nb);
         scatter_body<false>(s, cta);
         for (uint32_t r = w0; r < nb; r += warps) {
             block_neighbors<D, false>(s, r);

@@ -542,6 +542,11 @@ void destroy_graphs(slosh_ctx *c);
 // against separate kernels: 3D blobs of 30 k fluid particles 40 and 58, 97 k 56
 // and 66, 149 k 65 and 71, 195 k 76 and 75, 250 k 95 and 82 (sand the same
 // order); 2D dam breaks of 63 k 32 and 51, 154 k 54 and 61, 251 k 62 and 72.
+// Fluid particles thrown apart in 3D, by particles and active blocks: 20,000 in
+// 5,800 blocks 106 and 107, 60,000 in 39,000 525 and 574, 150,000 in 40,000 586
+// and 665, 20,000 in 36,000 421 and 409, 5,000 in 24,000 255 and 217: at several
+// blocks a particle the separate kernels' higher occupancy would still win, but
+// the host does not know the blocks without a wait.
 constexpr uint32_t STEPS_MAX_PARTICLES_3D = 180000, STEPS_MAX_PARTICLES_2D = 262144;
 // Substeps a launch takes at most, so that no launch holds the GPU for long.
 constexpr uint32_t STEPS_PER_LAUNCH = 32;

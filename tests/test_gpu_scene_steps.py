@@ -3,10 +3,13 @@ the separate kernels (SLOSH_SCENE_STEPS=0): the same bits.
 
 The scenes sit where the one-launch form can go wrong: one particle, a block
 that does not fit its sorting buffer (768 entries), more blocks than shared
-P2G takes (16 an SM) and a count that is no multiple of 32, cell widths that
+P2G takes (16 an SM) and a count that is no multiple of 32, more blocks than
+are ranked all against all (4,096), cell widths that
 are no power of two, two-way coupling, damping with several models, 2D; and
 more substeps than one launch holds (32), in one call and in several.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -41,6 +44,8 @@ def _scene(name):
         return _points(0.3 + rng.uniform(0.0, 3.9 / 64, (1000, 3)), 1 / 64, 3, elastic, rng.normal(0, 0.1, (1000, 3)))
     if name == "scattered":
         return _points(rng.uniform(0.1, 2.0, (2777, 3)), 1 / 64, 3, elastic, rng.normal(0, 1.0, (2777, 3)))
+    if name == "spread":
+        return _spread()
     if name == "fluid_odd":
         return _points(rng.uniform(0.1, 0.4, (4321, 2)), 1 / 50, 2, fluid, rng.normal(0, 0.5, (4321, 2)))
     if name == "two_way":
@@ -56,6 +61,13 @@ def _scene(name):
     return scenes.dam_break_2d(h=1 / 128)
 
 
+def _spread():
+    """Particles thrown apart: about 24,000 blocks for 5,000 particles."""
+    rng = np.random.default_rng(0)
+    model = ParticleModel.fluid_tait(1000.0, 1.0e4, 7.0)
+    return _points(rng.uniform(0.2, 2.2, (5000, 3)), 1 / 64, 3, model, rng.normal(0, 0.3, (5000, 3)))
+
+
 def _run(sc, monkeypatch, fused, calls):
     monkeypatch.setenv("SLOSH_SCENE_STEPS", "1" if fused else "0")
     data = scenes.build_mpm_data(sc)
@@ -68,7 +80,7 @@ def _run(sc, monkeypatch, fused, calls):
     return out, bodies, st, kernels
 
 
-@pytest.mark.parametrize("name", ["one", "dense_block", "scattered", "fluid_odd", "two_way", "models", "dam"])
+@pytest.mark.parametrize("name", ["one", "dense_block", "scattered", "spread", "fluid_odd", "two_way", "models", "dam"])
 def test_one_launch_matches_separate_kernels(cuda_lib, monkeypatch, name):
     sc = _scene(name)
     a, ab, ast, ak = _run(sc, monkeypatch, True, [1, 36])
@@ -78,6 +90,29 @@ def test_one_launch_matches_separate_kernels(cuda_lib, monkeypatch, name):
     assert ab.tobytes() == bb.tobytes()
     for k in ("n_blocks", "n_primary_blocks", "n_svd_fp64"):
         assert ast[k] == bst[k], k
+
+
+def test_spread_scene_is_linear_in_its_blocks(cuda_lib, monkeypatch):
+    """Ranking takes time linear in the blocks: a scene thrown apart costs the
+    one launch no more than three times the separate kernels (which are linear;
+    1.2 times measured, 13 times where all keys were compared)."""
+    sc = _spread()
+    best = {}
+    for fused in ("1", "0"):
+        monkeypatch.setenv("SLOSH_SCENE_STEPS", fused)
+        data, pipe = scenes.build_mpm_data(sc), MpmPipeline()
+        pipe.launch_step(data, 16)
+        data.sync()
+        times = []
+        for _ in range(5):
+            t0 = time.perf_counter()
+            pipe.launch_step(data, 16)
+            data.sync()
+            times.append(time.perf_counter() - t0)
+        best[fused] = min(times)
+        data.close()
+    print(f"16 substeps: one launch {best['1'] * 1e6:.0f} us, separate kernels {best['0'] * 1e6:.0f} us")
+    assert best["1"] <= 3.0 * best["0"]
 
 
 @pytest.mark.parametrize("reported_by", ["sync", "positions", "timestep_bound"])
