@@ -107,6 +107,14 @@ template <int D> struct CellLoc {
     int local[D];
 };
 
+// a b - c d and a b + c d with the contraction fixed.  A sum of two products
+// could be contracted to an FMA on either one, and a product with several uses
+// contracted or not; the compiler's choice may differ between the kernels a
+// function is inlined in.  These, and explicit FMAs, fix it, so that a stage
+// gives the same bits in its own kernel and inside k_scene_steps.
+__device__ __forceinline__ float products_diff(float a, float b, float c, float d) { return fmaf(a, b, -(c * d)); }
+__device__ __forceinline__ float products_sum(float a, float b, float c, float d) { return fmaf(a, b, c * d); }
+
 // x / h, correctly rounded.  When h is a power of two its reciprocal is
 // exact and x * (1/h) is the same correctly rounded quotient, so the IEEE
 // division is replaced by a multiplication without changing any bit.
@@ -281,15 +289,22 @@ constexpr double IMPULSE_UNITS = 1099511627776.0;  // 2^40
 // Rotation matrix of the unit quaternion q = (i, j, k, w).
 __host__ __device__ inline void quat_matrix(const float *q, float (&R)[3][3]) {
     const float x = q[0], y = q[1], z = q[2], w = q[3];
-    R[0][0] = 1.f - 2.f * (y * y + z * z);
-    R[0][1] = 2.f * (x * y - z * w);
-    R[0][2] = 2.f * (x * z + y * w);
-    R[1][0] = 2.f * (x * y + z * w);
-    R[1][1] = 1.f - 2.f * (x * x + z * z);
-    R[1][2] = 2.f * (y * z - x * w);
-    R[2][0] = 2.f * (x * z - y * w);
-    R[2][1] = 2.f * (y * z + x * w);
-    R[2][2] = 1.f - 2.f * (x * x + y * y);
+#ifdef __CUDA_ARCH__
+    auto sum = [](float a, float b, float c, float d) { return products_sum(a, b, c, d); };
+    auto diff = [](float a, float b, float c, float d) { return products_diff(a, b, c, d); };
+#else
+    auto sum = [](float a, float b, float c, float d) { return a * b + c * d; };
+    auto diff = [](float a, float b, float c, float d) { return a * b - c * d; };
+#endif
+    R[0][0] = 1.f - 2.f * sum(y, y, z, z);
+    R[0][1] = 2.f * diff(x, y, z, w);
+    R[0][2] = 2.f * sum(x, z, y, w);
+    R[1][0] = 2.f * sum(x, y, z, w);
+    R[1][1] = 1.f - 2.f * sum(x, x, z, z);
+    R[1][2] = 2.f * diff(y, z, x, w);
+    R[2][0] = 2.f * diff(x, z, y, w);
+    R[2][1] = 2.f * sum(y, z, x, w);
+    R[2][2] = 1.f - 2.f * sum(x, x, y, y);
 }
 
 // out = R M R^T (rot = true) or R^T M R (rot = false) for 3 x 3 M.

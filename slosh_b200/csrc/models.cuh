@@ -59,7 +59,7 @@ template <> struct SvdD<2> {
 
 template <int D> __device__ __forceinline__ float det(const float (&F)[D][D]) {
     if constexpr (D == 3) {
-        // contraction fixed, as products_diff in transfer.cuh
+        // contraction fixed, as products_diff
         const float c0 = fmaf(F[1][1], F[2][2], -(F[1][2] * F[2][1])), c1 = fmaf(F[1][0], F[2][2], -(F[1][2] * F[2][0])),
                     c2 = fmaf(F[1][0], F[2][1], -(F[1][1] * F[2][0]));
         return fmaf(F[0][2], c2, fmaf(F[0][0], c0, -(F[0][1] * c1)));

@@ -443,15 +443,6 @@ template <int D> __global__ void __launch_bounds__(P2G_ATOMIC_THREADS, 4) k_p2g_
 // Colliders: Sim3/Sim2 poses, ball and cuboid projections, collide() and the
 // boundary-condition projection.
 // ---------------------------------------------------------------------------
-//
-// A sum of two products could be contracted to an FMA on either one, and a
-// product with several uses contracted or not; the compiler's choice may differ
-// between the kernels a function is inlined in.  products_sum, products_diff
-// and explicit roundings fix it, so that a stage gives the same bits in its
-// own kernel and inside k_scene_steps.
-__device__ __forceinline__ float products_diff(float a, float b, float c, float d) { return fmaf(a, b, -(c * d)); }
-__device__ __forceinline__ float products_sum(float a, float b, float c, float d) { return fmaf(a, b, c * d); }
-
 __device__ __forceinline__ void quat_rotate(const float *q, const float *v, float *out) {
     const float t0 = 2.f * products_diff(q[1], v[2], q[2], v[1]);
     const float t1 = 2.f * products_diff(q[2], v[0], q[0], v[2]);
@@ -568,7 +559,7 @@ __device__ __forceinline__ bool capsule_boundary(const float *a, const float *b,
 // (cylinder.slang:72-125): inside, the nearest of the two caps and the
 // side; outside, the cap disc, the cap rim or the side.  Returns "inside".
 __device__ __forceinline__ bool cylinder_boundary(float hh, float r, const float *p, float *out) {
-    const float rxz = sqrtf(p[0] * p[0] + p[2] * p[2]);
+    const float rxz = sqrtf(products_sum(p[0], p[0], p[2], p[2]));
     const float dx = rxz > 0.f ? p[0] / rxz : 1.f, dz = rxz > 0.f ? p[2] / rxz : 0.f;
     const float sx = dx * r, sz = dz * r;
     if (p[1] >= -hh && p[1] <= hh && rxz <= r) {
@@ -597,7 +588,7 @@ __device__ __forceinline__ bool cylinder_boundary(float hh, float r, const float
 // point of the generatrix through the point's azimuth, or (inside) the base
 // when that is nearer.  Returns "inside".
 __device__ __forceinline__ bool cone_boundary(float hh, float r, const float *p, float *out) {
-    const float rxz = sqrtf(p[0] * p[0] + p[2] * p[2]);
+    const float rxz = sqrtf(products_sum(p[0], p[0], p[2], p[2]));
     const float dx = rxz > 0.f ? p[0] / rxz : 1.f, dz = rxz > 0.f ? p[2] / rxz : 0.f;
     const float base[3] = {p[0], -hh, p[2]};
     if (p[1] < -hh && rxz <= r) {
@@ -612,10 +603,11 @@ __device__ __forceinline__ bool cone_boundary(float hh, float r, const float *p,
     const float gen[3] = {rim[0] - apex[0], rim[1] - apex[1], rim[2] - apex[2]};
     const float ap[3] = {p[0] - apex[0], p[1] - apex[1], p[2] - apex[2]};
     const float axis[3] = {0.f, -2.0f * hh, 0.f};
-    const float c1[3] = {gen[1] * ap[2] - gen[2] * ap[1], gen[2] * ap[0] - gen[0] * ap[2], gen[0] * ap[1] - gen[1] * ap[0]};
-    const float c2[3] = {gen[1] * axis[2] - gen[2] * axis[1], gen[2] * axis[0] - gen[0] * axis[2],
-                         gen[0] * axis[1] - gen[1] * axis[0]};
-    const bool in = p[1] >= -hh && p[1] <= hh && (c1[0] * c2[0] + c1[1] * c2[1] + c1[2] * c2[2]) >= 0.f;
+    const float c1[3] = {products_diff(gen[1], ap[2], gen[2], ap[1]), products_diff(gen[2], ap[0], gen[0], ap[2]),
+                         products_diff(gen[0], ap[1], gen[1], ap[0])};
+    const float c2[3] = {products_diff(gen[1], axis[2], gen[2], axis[1]), products_diff(gen[2], axis[0], gen[0], axis[2]),
+                         products_diff(gen[0], axis[1], gen[1], axis[0])};
+    const bool in = p[1] >= -hh && p[1] <= hh && fmaf(c1[2], c2[2], products_sum(c1[0], c2[0], c1[1], c2[1])) >= 0.f;
     if (in) {
         float d_side = 0.f, d_base = 0.f;
 #pragma unroll
@@ -652,19 +644,19 @@ __device__ __forceinline__ bool project_on_boundary(const DevBody &b, const floa
             outp[i] = local[i] + shift;
             const float sw = (local[i] > 0.f) ? 1.f : ((local[i] < 0.f) ? -1.f : 0.f);
             sgn[i] = sw + (fabsf(sw) - 1.f);
-            diff[i] = b.sa[i] - sgn[i] * local[i];
+            diff[i] = fmaf(-sgn[i], local[i], b.sa[i]);
             inp[i] = local[i];
             in = in && (local[i] == outp[i]);
         }
         if constexpr (D == 3) {
             const bool px = diff[0] <= diff[1] && diff[0] <= diff[2];
             const bool py = diff[1] <= diff[0] && diff[1] <= diff[2];
-            if (px) inp[0] = local[0] + diff[0] * sgn[0];
-            else if (py) inp[1] = local[1] + diff[1] * sgn[1];
-            else inp[2] = local[2] + diff[2] * sgn[2];
+            if (px) inp[0] = fmaf(diff[0], sgn[0], local[0]);
+            else if (py) inp[1] = fmaf(diff[1], sgn[1], local[1]);
+            else inp[2] = fmaf(diff[2], sgn[2], local[2]);
         } else {
-            if (diff[0] <= diff[1]) inp[0] = local[0] + diff[0] * sgn[0];
-            else inp[1] = local[1] + diff[1] * sgn[1];
+            if (diff[0] <= diff[1]) inp[0] = fmaf(diff[0], sgn[0], local[0]);
+            else inp[1] = fmaf(diff[1], sgn[1], local[1]);
         }
 #pragma unroll
         for (int i = 0; i < D; ++i) lp[i] = in ? inp[i] : outp[i];

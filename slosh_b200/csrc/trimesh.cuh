@@ -206,7 +206,7 @@ __device__ __forceinline__ void triangle_closest(const float3 a, const float3 b,
                                                  float3 &q, uint32_t &feat, uint32_t &fid) {
     const float3 ab = make_float3(b.x - a.x, b.y - a.y, b.z - a.z), ac = make_float3(c.x - a.x, c.y - a.y, c.z - a.z);
     const float3 ap = make_float3(p.x - a.x, p.y - a.y, p.z - a.z);
-    auto dot3 = [](float3 u, float3 w) { return u.x * w.x + u.y * w.y + u.z * w.z; };
+    auto dot3 = [](float3 u, float3 w) { return fmaf(u.z, w.z, products_sum(u.x, w.x, u.y, w.y)); };
     const float d1 = dot3(ab, ap), d2 = dot3(ac, ap);
     if (d1 <= 0.f && d2 <= 0.f) {
         q = a, feat = 0, fid = 0;
@@ -218,10 +218,10 @@ __device__ __forceinline__ void triangle_closest(const float3 a, const float3 b,
         q = b, feat = 0, fid = 1;
         return;
     }
-    const float vc = d1 * d4 - d3 * d2;
+    const float vc = products_diff(d1, d4, d3, d2);
     if (vc <= 0.f && d1 >= 0.f && d3 <= 0.f) {
         const float t = d1 / (d1 - d3);
-        q = make_float3(a.x + t * ab.x, a.y + t * ab.y, a.z + t * ab.z), feat = 1, fid = 0;
+        q = make_float3(fmaf(t, ab.x, a.x), fmaf(t, ab.y, a.y), fmaf(t, ab.z, a.z)), feat = 1, fid = 0;
         return;
     }
     const float3 cp = make_float3(p.x - c.x, p.y - c.y, p.z - c.z);
@@ -230,22 +230,23 @@ __device__ __forceinline__ void triangle_closest(const float3 a, const float3 b,
         q = c, feat = 0, fid = 2;
         return;
     }
-    const float vb = d5 * d2 - d1 * d6;
+    const float vb = products_diff(d5, d2, d1, d6);
     if (vb <= 0.f && d2 >= 0.f && d6 <= 0.f) {
         const float t = d2 / (d2 - d6);
-        q = make_float3(a.x + t * ac.x, a.y + t * ac.y, a.z + t * ac.z), feat = 1, fid = 2;
+        q = make_float3(fmaf(t, ac.x, a.x), fmaf(t, ac.y, a.y), fmaf(t, ac.z, a.z)), feat = 1, fid = 2;
         return;
     }
-    const float va = d3 * d6 - d5 * d4;
+    const float va = products_diff(d3, d6, d5, d4);
     if (va <= 0.f && (d4 - d3) >= 0.f && (d5 - d6) >= 0.f) {
         const float t = (d4 - d3) / ((d4 - d3) + (d5 - d6));
-        q = make_float3(b.x + t * (c.x - b.x), b.y + t * (c.y - b.y), b.z + t * (c.z - b.z)), feat = 1, fid = 1;
+        q = make_float3(fmaf(t, c.x - b.x, b.x), fmaf(t, c.y - b.y, b.y), fmaf(t, c.z - b.z, b.z)), feat = 1, fid = 1;
         return;
     }
     const float den = va + vb + vc;
     if (den != 0.f) {
         const float inv = 1.f / den, v = vb * inv, w = vc * inv;
-        q = make_float3(a.x + ab.x * v + ac.x * w, a.y + ab.y * v + ac.y * w, a.z + ab.z * v + ac.z * w);
+        q = make_float3(fmaf(ac.x, w, fmaf(ab.x, v, a.x)), fmaf(ac.y, w, fmaf(ab.y, v, a.y)),
+                        fmaf(ac.z, w, fmaf(ab.z, v, a.z)));
     } else {
         q = a;  // degenerate triangle
     }
@@ -276,7 +277,7 @@ __device__ __forceinline__ bool trimesh_project(const TriMeshRef &m, const float
             triangle_closest(make_float3(a4.x, a4.y, a4.z), make_float3(b4.x, b4.y, b4.z),
                              make_float3(c4.x, c4.y, c4.z), pt, q, feat, fid);
             const float dx = q.x - pt.x, dy = q.y - pt.y, dz = q.z - pt.z;
-            const float dist = sqrtf(dx * dx + dy * dy + dz * dz);
+            const float dist = sqrtf(fmaf(dz, dz, products_sum(dx, dx, dy, dy)));
             if (dist <= best) {
                 best = dist, bq = q, bfeat = feat, bfid = fid, btri = t;
                 found = true;
@@ -287,7 +288,7 @@ __device__ __forceinline__ bool trimesh_project(const TriMeshRef &m, const float
             const float sx = fmaxf(mn.x - pt.x, 0.f) - fmaxf(pt.x - mx.x, 0.f);
             const float sy = fmaxf(mn.y - pt.y, 0.f) - fmaxf(pt.y - mx.y, 0.f);
             const float sz = fmaxf(mn.z - pt.z, 0.f) - fmaxf(pt.z - mx.z, 0.f);
-            curr = sqrtf(sx * sx + sy * sy + sz * sz) < best ? entry : exit;
+            curr = sqrtf(fmaf(sz, sz, products_sum(sx, sx, sy, sy))) < best ? entry : exit;
         }
     }
     if (!found) return false;
@@ -303,9 +304,10 @@ __device__ __forceinline__ bool trimesh_project(const TriMeshRef &m, const float
                      c4 = vtx[vbase + idx[tbase + 3u * btri + 2u]];
         const float3 ab = make_float3(b4.x - a4.x, b4.y - a4.y, b4.z - a4.z),
                      ac = make_float3(c4.x - a4.x, c4.y - a4.y, c4.z - a4.z);
-        pn = make_float3(ab.y * ac.z - ab.z * ac.y, ab.z * ac.x - ab.x * ac.z, ab.x * ac.y - ab.y * ac.x);
+        pn = make_float3(products_diff(ab.y, ac.z, ab.z, ac.y), products_diff(ab.z, ac.x, ab.x, ac.z),
+                         products_diff(ab.x, ac.y, ab.y, ac.x));
     }
-    inside = pn.x * (pt.x - bq.x) + pn.y * (pt.y - bq.y) + pn.z * (pt.z - bq.z) <= 0.f;
+    inside = fmaf(pn.z, pt.z - bq.z, products_sum(pn.x, pt.x - bq.x, pn.y, pt.y - bq.y)) <= 0.f;
     out[0] = bq.x, out[1] = bq.y, out[2] = bq.z;
     return true;
 }

@@ -6,7 +6,9 @@ that does not fit its sorting buffer (768 entries), more blocks than shared
 P2G takes (16 an SM) and a count that is no multiple of 32, more blocks than
 are ranked all against all (4,096), cell widths that
 are no power of two, two-way coupling, damping with several models, 2D; and
-more substeps than one launch holds (32), in one call and in several.
+more substeps than one launch holds (32), in one call and in several.  Every
+collider shape and every model in both dimensions: what one kernel contracts to
+an FMA, the other has to.
 """
 import time
 
@@ -21,7 +23,10 @@ from slosh_b200.pipeline import (
     RigidBody,
     SimulationParams,
     SloshError,
+    box_mesh,
+    heightfield_mesh,
     make_particles,
+    quat_from_axis_angle,
 )
 
 pytestmark = pytest.mark.gpu
@@ -78,6 +83,72 @@ def _run(sc, monkeypatch, fused, calls):
     kernels = data.kernels_per_substep
     data.close()
     return out, bodies, st, kernels
+
+
+MODELS = {
+    "elastic": ParticleModel.elastic(1.0e5, 0.3),
+    "neo_hookean": ParticleModel.elastic_neo_hookean(1.0e5, 0.3),
+    "sand": ParticleModel.sand(1.0e5, 0.3, friction_angle_deg=30.0),
+    "sand_neo_hookean": ParticleModel.sand_neo_hookean(1.0e5, 0.3),
+    "fluid": ParticleModel.fluid_tait(1000.0, 1.0e4, 7.0),
+}
+_HEIGHTS = 0.03 * np.sin(np.arange(20.0)).reshape(4, 5)
+SHAPES = {
+    "ball": (3, ("ball", 0.06), "two_way"),
+    "cuboid": (3, ("cuboid", (0.05, 0.07, 0.04)), "two_way"),
+    "capsule": (3, ("capsule", ((-0.05, 0.01, 0.0), (0.06, 0.0, 0.02), 0.04)), "one_way"),
+    "cylinder": (3, ("cylinder", (0.05, 0.06)), "one_way"),
+    "cone": (3, ("cone", (0.06, 0.05)), "one_way"),
+    "box_mesh": (3, ("trimesh", box_mesh((0.06, 0.04, 0.05))), "one_way"),
+    "height_mesh": (3, ("trimesh", heightfield_mesh(_HEIGHTS, (0.3, 0.3))), "one_way"),
+    "ball_2d": (2, ("ball", 0.06), "two_way"),
+    "cuboid_2d": (2, ("cuboid", (0.05, 0.07)), "two_way"),
+    "capsule_2d": (2, ("capsule", ((-0.05, 0.01), (0.06, 0.0), 0.04)), "one_way"),
+}
+
+
+def _cloud(dim, k, model, body=None):
+    """Particles at random about (0.5, ...), moving and a little strained, and
+    a body turning among them."""
+    rng = np.random.default_rng(11)
+    pts = rng.uniform(0.38, 0.62, (3001 if dim == 3 else 1501, dim))
+    sc = _points(pts, 1.0 / k, dim, model, rng.normal(0.0, 0.4, pts.shape))
+    if model.tag != 4:  # a fluid keeps its volume ratio alone
+        f = np.eye(dim) + rng.normal(0.0, 0.02, (len(pts), dim, dim))
+        for r in range(dim):
+            for c in range(dim):
+                sc.particles["def_grad"][:, c * 3 + r] = f[:, r, c]
+    if body is not None:
+        shape, coupling = body
+        kw = dict(translation=(0.5,) * dim, rotation=quat_from_axis_angle((0.3, 1.0, 0.2), 0.4) if dim == 3 else 0.4,
+                  linvel=(0.1, -0.2, 0.15)[:dim], angvel=(0.3, -0.5, 0.4) if dim == 3 else (0.7,))
+        sc.bodies.insert(0, RigidBody.two_way(shape, 800.0, dim, **kw) if coupling == "two_way" else RigidBody(shape, **kw))
+    return sc
+
+
+@pytest.mark.parametrize("shape", list(SHAPES))
+def test_collider_bits_do_not_depend_on_the_kernel(cuda_lib, monkeypatch, shape):
+    dim, what, coupling = SHAPES[shape]
+    sc = _cloud(dim, 64, MODELS["neo_hookean"], (what, coupling))
+    a, ab, _, ak = _run(sc, monkeypatch, True, [12])
+    b, bb, _, bk = _run(sc, monkeypatch, False, [12])
+    assert ak == 1 and bk > 1
+    assert a.tobytes() == b.tobytes()
+    assert ab.tobytes() == bb.tobytes()
+    alone, _, _, _ = _run(_cloud(dim, 64, MODELS["neo_hookean"]), monkeypatch, True, [12])
+    assert a["velocity"].tobytes() != alone["velocity"].tobytes(), "the body was met"
+
+
+@pytest.mark.parametrize("k", [64, 56])
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("model", list(MODELS))
+def test_model_bits_do_not_depend_on_the_kernel(cuda_lib, monkeypatch, model, dim, k):
+    sc = _cloud(dim, k, MODELS[model])
+    a, _, ast, ak = _run(sc, monkeypatch, True, [12])
+    b, _, bst, bk = _run(sc, monkeypatch, False, [12])
+    assert ak == 1 and bk > 1
+    assert a.tobytes() == b.tobytes()
+    assert ast["n_svd_fp64"] == bst["n_svd_fp64"]
 
 
 @pytest.mark.parametrize("name", ["one", "dense_block", "scattered", "spread", "fluid_odd", "two_way", "models", "dam"])
