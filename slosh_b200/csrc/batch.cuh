@@ -816,7 +816,8 @@ int slosh_batch_download_positions(slosh_batch *b, uint32_t slot, float *out, ui
     if (n > 0) {
         DevScene s = make_batch_scene(b, c->parity);
         float4 *tmp = (float4 *)c->staging;  // staging holds >= 12 float4 per particle of the largest scene
-        k_positions<true><<<grid_for(scene_span(b, sl), 256, (uint32_t)c->sm_count * 16), 256, 0, st>>>(s, tmp, slot, scene_start(b, sl), scene_span(b, sl));
+        const uint32_t start = scene_start(b, sl), span = scene_span(b, sl);
+        k_positions<true><<<grid_for(span, 256, (uint32_t)c->sm_count * 16), 256, 0, st>>>(s, tmp, slot, start, span);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(out, tmp, (size_t)n * 16, cudaMemcpyDeviceToHost, st));
     }
@@ -844,15 +845,22 @@ int slosh_batch_timestep_bound(slosh_batch *b, uint32_t slot, float *dt_out, voi
     cudaStream_t st = pick(c, stream);
     const DevScene s = make_batch_scene(b, c->parity);
     uint32_t *out = c->small + 3;
-    CK(cudaMemsetAsync(out, 0xff, 4, st));
     const slosh_batch::Slot &sl = b->slots[slot];
-    const uint32_t g = grid_for(scene_span(b, sl), 256, (uint32_t)c->sm_count * 16);
-    if (c->dim == 3) k_timestep_bound<3, true><<<g, 256, 0, st>>>(s, slot, scene_start(b, sl), scene_span(b, sl), out);
-    else k_timestep_bound<2, true><<<g, 256, 0, st>>>(s, slot, scene_start(b, sl), scene_span(b, sl), out);
-    CK(cudaGetLastError());
     uint32_t u = 0;
-    CK(cudaMemcpyAsync(&u, out, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    for (;;) {
+        CK(cudaMemsetAsync(out, 0xff, 4, st));
+        const uint32_t start = scene_start(b, sl), span = scene_span(b, sl), g = grid_for(span, 256, (uint32_t)c->sm_count * 16);
+        if (c->dim == 3) k_timestep_bound<3, true><<<g, 256, 0, st>>>(s, slot, start, span, out);
+        else k_timestep_bound<2, true><<<g, 256, 0, st>>>(s, slot, start, span, out);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(&u, out, 4, cudaMemcpyDeviceToHost, st));
+        uint32_t e = 0;
+        if (int r = wait_and_read_error(c, st, &e)) return r;
+        if (e == 0u || b->misplaced) break;
+        // an error that is still to be reported: storage may have lost
+        // particles, so the scene may lie elsewhere
+        b->misplaced = true;
+    }
     *dt_out = (float)u / TIMESTEP_FLOAT_TO_INT;
     return SLOSH_OK;
 }

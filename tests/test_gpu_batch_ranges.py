@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from slosh_b200 import scenes
+from slosh_b200._lib import SLOSH_E_OVERFLOW, SloshError
 from slosh_b200.batch import MpmBatch
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,25 @@ def test_reads_follow_scenes_that_leave_and_join(cuda_lib):
     check()
     for x in [b, *alone]:
         x.close()
+
+
+def test_timestep_bound_after_an_unreported_overflow(cuda_lib):
+    """More blocks than the pool's grid holds: particles are lost, and the
+    scenes behind move down in storage.  The bound counts every particle left
+    to its scene, whether or not the overflow was reported yet."""
+    nothing = 4.294967e-3  # of a scene without particles
+    survived = False
+    for _ in range(10):  # which blocks find room differs from run to run
+        b = MpmBatch(3, max_particles=1 << 17, grid_capacity=128, max_scenes=16, max_bodies=32)
+        b.add(scenes.random_scene_3d(60000, "fluid", 1 / 64, seed=1))
+        slots = [b.add(scenes.random_scene_3d(600, "fluid", 1 / 64, seed=2 + i)) for i in range(8)]
+        b.step(1)
+        before = [b.timestep_bound(s) for s in slots]
+        with pytest.raises(SloshError) as e:
+            b.sync()
+        assert e.value.code == SLOSH_E_OVERFLOW
+        after = [b.timestep_bound(s) for s in slots]
+        b.close()
+        assert before == after
+        survived = survived or min(after) < 0.9 * nothing
+    assert survived, "a small scene kept particles"
