@@ -593,8 +593,9 @@ cudaError_t enqueue_scene_steps(slosh_ctx *c, uint32_t n, cudaStream_t st) {
 }
 
 // Prepares the kernels of dimension D; false when the device cannot hold a
-// cooperative launch of one CTA an SM.
-template <int D> bool scene_steps_fit(const slosh_ctx *c) {
+// cooperative launch of one CTA an SM.  At every context's creation: the
+// attribute belongs to the CUDA context, which may have been reset since.
+template <int D> bool scene_steps_fit() {
     bool ok = true;
     auto one = [&](auto pow2, auto model) {
         auto *k = k_scene_steps<D, decltype(pow2)::value, decltype(model)::value>;
@@ -613,20 +614,6 @@ template <int D> bool scene_steps_fit(const slosh_ctx *c) {
     if (!ok) cudaGetLastError();
     return ok;
 }
-// The same, once for each device and dimension of the process (loading and
-// querying five kernels takes milliseconds).
-bool scene_steps_ready(const slosh_ctx *c) {
-    static std::mutex mutex;
-    static std::map<std::pair<int, int>, bool> known;
-    std::lock_guard<std::mutex> lock(mutex);
-    const auto key = std::make_pair(c->device, c->dim);
-    const auto it = known.find(key);
-    if (it != known.end()) return it->second;
-    const bool ok = c->dim == 3 ? scene_steps_fit<3>(c) : scene_steps_fit<2>(c);
-    known[key] = ok;
-    return ok;
-}
-
 // Sets whether substeps keep their grid, from the mode and the particle
 // count; the graphs are rebuilt when that changes.
 void update_reuse(slosh_ctx *c) {
@@ -1068,7 +1055,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
     int coop = 0;
     c->scene_steps = c->scene_steps &&
                      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) == cudaSuccess && coop &&
-                     scene_steps_ready(c);
+                     (c->dim == 3 ? scene_steps_fit<3>() : scene_steps_fit<2>());
     c->reuse_mode = 2u;
     if (const char *r = std::getenv("SLOSH_GRID_REUSE")) c->reuse_mode = std::strcmp(r, "0") == 0 ? 0u : 1u;
     update_reuse(c);
