@@ -441,7 +441,7 @@ int slosh_batch_create(const slosh_batch_config *cfg, slosh_batch **out) {
         (st = dalloc(c, &c->coll[1], (size_t)cap * 64)) || (st = dalloc(c, &c->coll_id[0], (size_t)cap * 64)) ||
         (st = dalloc(c, &c->coll_id[1], (size_t)cap * 64)) || (st = dalloc(c, &c->bodies, b->max_bodies)) ||
         (st = dalloc(c, &c->body_imp, (size_t)b->max_bodies * 6)) ||
-        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 1)) || (st = dalloc(c, &c->small, 4)) ||
+        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 2)) || (st = dalloc(c, &c->small, 4)) ||
         (st = dalloc(c, &b->scene_nblk, b->max_scenes)) || (st = dalloc(c, &b->scene_bbase, b->max_scenes)) ||
         (st = dalloc(c, &b->scene_fill, b->max_scenes)) || (st = dalloc(c, &b->scenes_dev, b->max_scenes)) ||
         (st = dalloc(c, &b->n_dev, 1)) || (st = dalloc(c, &b->g2p_lists, (size_t)G2P_CLASSES * cap)) ||
@@ -454,7 +454,7 @@ int slosh_batch_create(const slosh_batch_config *cfg, slosh_batch **out) {
     cudaMemset(c->hvals[1], 0xff, (size_t)hcap * 4);
     cudaMemset(c->slot_counts, 0, (size_t)hcap * CELLS * 4);
     cudaMemset(c->ctr, 0, sizeof(Counters));
-    cudaMemset(c->err, 0, 4);
+    cudaMemset(c->err, 0, 8);
     cudaMemset(c->small, 0, 16);
     cudaMemset(c->body_imp, 0, (size_t)b->max_bodies * 6 * sizeof(unsigned long long));
 

@@ -3,8 +3,8 @@
 // A scene of tens of thousands of particles has one or two blocks an SM: each
 // stage of the substep is a few microseconds of latency, and launching the
 // stages one after another (13 kernels in a graph) costs more than running
-// them.  Here one CTA an SM runs all stages of several substeps, with a grid
-// barrier where a stage needs the whole grid's results of the one before:
+// them.  Here up to one CTA an SM runs all stages of several substeps, with a
+// grid barrier where a stage needs the whole grid's results of the one before:
 //
 //   touch     particles counted per cell, their blocks and the blocks' +1
 //             neighbours inserted                       (k_touch, k_neighbors)
@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(STEPS_THREADS, 1)
         if (blockIdx.x == gridDim.x - 1u && warp == STEPS_THREADS / 32 - 1) {
             if (lane < s.n_bodies) move_body<D>(s, lane);
             if (lane == 0) {
+                s.err[1] = nb;
                 s.ctr->last_n_blocks = nb;
                 s.ctr->last_n_primary = s.ctr->n_primary;
                 s.ctr->n_primary = 0u;

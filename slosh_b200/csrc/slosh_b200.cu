@@ -108,7 +108,8 @@ struct slosh_ctx {
     uint32_t *mesh_idx = nullptr;
     uint32_t n_meshes = 0;
     Counters *ctr = nullptr;
-    uint32_t *err = nullptr;
+    uint32_t *err = nullptr;    // [0] error bits, [1] active blocks of the last one-launch substep
+    uint32_t blocks_seen = 0;   // err[1] at the last wait (0: none since the upload)
     uint32_t *small = nullptr;  // [0] n_mat, [1] scene flags, [2] debug total
     uint32_t parity = 0;
     // A one-launch substep gave up waiting: the launch ended in mid-substep and
@@ -551,6 +552,26 @@ constexpr uint32_t STEPS_MAX_PARTICLES_3D = 180000, STEPS_MAX_PARTICLES_2D = 262
 // Substeps a launch takes at most, so that no launch holds the GPU for long.
 constexpr uint32_t STEPS_PER_LAUNCH = 32;
 
+// CTAs of a launch: an SM's whole shared memory each, so what a scene does not
+// need is left to scenes on other streams.  About one CTA a full block, and two
+// active blocks, from 32 on: every SM from 24,700 particles or 300 blocks, and
+// while no wait has brought the scene's block count back yet (a scene thrown
+// apart needs the SMs at any size: 5,000 particles in 24,000 blocks 255 us on
+// 148 CTAs, 830 on 32).  Microseconds a substep on every SM and on these CTAs:
+// 3,375 sand particles 38.8 and 38.5 (32 CTAs), 8,000 39.1 and 38.7 (50), 10,648
+// 40.0 and 40.6 (64), 15,625 40.3 and 40.8 (94); larger scenes need the SMs
+// (59,319 fluid particles 43 on 148, 52 on 111, 55 on 74).  Two and four scenes
+// of 8,000 fluid particles on as many streams: 73 and 146 where each takes every
+// SM, 38 and 75 on 74 CTAs, 70 and 99 as separate kernels.
+constexpr uint32_t STEPS_PARTICLES_PER_CTA = 168, STEPS_BLOCKS_PER_CTA = 2, STEPS_MIN_CTAS = 32;
+uint32_t steps_grid(const slosh_ctx *c) {
+    const uint32_t all = (uint32_t)c->sm_count;
+    if (c->blocks_seen == 0) return all;
+    const uint32_t want = std::max((c->n + STEPS_PARTICLES_PER_CTA - 1) / STEPS_PARTICLES_PER_CTA,
+                                   (c->blocks_seen + STEPS_BLOCKS_PER_CTA - 1) / STEPS_BLOCKS_PER_CTA);
+    return std::min(all, std::max(want, STEPS_MIN_CTAS));
+}
+
 bool takes_scene_steps(const slosh_ctx *c) {
     return c->scene_steps && !c->reuse && c->p2g_variant == 0 &&
            c->n < (c->dim == 3 ? STEPS_MAX_PARTICLES_3D : STEPS_MAX_PARTICLES_2D);
@@ -562,7 +583,7 @@ cudaError_t launch_scene_steps(slosh_ctx *c, const ScenePair &pair, uint32_t n, 
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((uint32_t)c->sm_count);
+    cfg.gridDim = dim3(steps_grid(c));
     cfg.blockDim = dim3(STEPS_THREADS);
     cfg.dynamicSmemBytes = sizeof(StepsSmem<D>);
     cfg.stream = st;
@@ -593,7 +614,7 @@ cudaError_t enqueue_scene_steps(slosh_ctx *c, uint32_t n, cudaStream_t st) {
 }
 
 // Prepares the kernels of dimension D; false when the device cannot hold a
-// cooperative launch of one CTA an SM.  At every context's creation: the
+// cooperative launch of up to one CTA an SM.  At every context's creation: the
 // attribute belongs to the CUDA context, which may have been reset since.
 template <int D> bool scene_steps_fit() {
     bool ok = true;
@@ -855,10 +876,14 @@ int check_device_error(slosh_ctx *c) {
 
 // Waits for the stream's work and reads the error bits with the same wait:
 // the end of every download (a copy of its own after the wait was a second
-// round trip of about 10 us).
+// round trip of about 10 us).  The word behind them says how many blocks the
+// scene has, for the next launches' CTAs.
 int wait_and_read_error(slosh_ctx *c, cudaStream_t st, uint32_t *e) {
-    CK(cudaMemcpyAsync(e, c->err, 4, cudaMemcpyDeviceToHost, st));
+    uint32_t w[2] = {0, 0};
+    CK(cudaMemcpyAsync(w, c->err, 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    *e = w[0];
+    c->blocks_seen = w[1];
     return SLOSH_OK;
 }
 int wait_and_check(slosh_ctx *c, cudaStream_t st) {
@@ -1019,7 +1044,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
         (st = dalloc(c, &c->coll[1], (size_t)cap * 64)) || (st = dalloc(c, &c->coll_id[0], (size_t)cap * 64)) ||
         (st = dalloc(c, &c->coll_id[1], (size_t)cap * 64)) || (st = dalloc(c, &c->bodies, MAX_BODIES)) ||
         (st = dalloc(c, &c->body_imp, (size_t)MAX_BODIES * 6)) ||
-        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 1)) || (st = dalloc(c, &c->small, 4)) ||
+        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 2)) || (st = dalloc(c, &c->small, 4)) ||
         (st = dalloc(c, &c->staging, N)) || (st = dalloc(c, &c->bfirst2, cap)) || (st = dalloc(c, &c->bnp2, cap)) ||
         (st = dalloc(c, &c->bcell2, (size_t)cap * CELLS)) || (st = dalloc(c, &c->cell_delta, (size_t)cap * CELLS)) ||
         (st = dalloc(c, &c->touch, cap)) || (st = dalloc(c, &c->cur_touch, cap)) ||
@@ -1031,7 +1056,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
     cudaMemset(c->hvals[0], 0xff, hcap * 4);
     cudaMemset(c->hvals[1], 0xff, hcap * 4);
     cudaMemset(c->ctr, 0, sizeof(Counters));
-    cudaMemset(c->err, 0, 4);
+    cudaMemset(c->err, 0, 8);
     cudaMemset(c->slot_counts, 0, (size_t)hcap * CELLS * 4);
     cudaMemset(c->slot_total, 0, (size_t)hcap * 4);
     cudaMemset(c->body_imp, 0, (size_t)MAX_BODIES * 6 * sizeof(unsigned long long));
@@ -1099,7 +1124,7 @@ int slosh_upload_particles(slosh_ctx *c, const slosh_particle *particles, uint32
     CK(cudaMemcpyAsync(c->staging, particles, (size_t)n * sizeof(slosh_particle), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(c->mat_hkeys, 0xff, MAT_HASH * 4, st));
     CK(cudaMemsetAsync(c->small, 0, 16, st));
-    CK(cudaMemsetAsync(c->err, 0, 4, st));
+    CK(cudaMemsetAsync(c->err, 0, 8, st));
     CK(cudaMemsetAsync(c->ctr, 0, sizeof(Counters), st));
     if (int r = force_grid_rebuild(c, st)) return r;
     for (int k = 0; k < 2; ++k) {
@@ -1113,6 +1138,7 @@ int slosh_upload_particles(slosh_ctx *c, const slosh_particle *particles, uint32
     CK(cudaMemsetAsync(c->body_imp, 0, (size_t)MAX_BODIES * 6 * sizeof(unsigned long long), st));
     c->parity = 0;
     c->lost = false;
+    c->blocks_seen = 0;
     if (n > 0) {
         DevScene s = make_scene(c, 0, false);
         IoBuffers io{};

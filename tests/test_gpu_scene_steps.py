@@ -186,6 +186,33 @@ def test_spread_scene_is_linear_in_its_blocks(cuda_lib, monkeypatch):
     assert best["1"] <= 3.0 * best["0"]
 
 
+def test_small_scenes_on_two_streams_share_the_gpu(cuda_lib):
+    """A launch takes the SMs its scene needs, once a wait has brought its block
+    count back: two scenes of 8,000 particles,
+    each on its own stream, are stepped in less than the sum of their times
+    (1.04 times one scene's measured; 2.0 where each took every SM)."""
+    data = [scenes.build_mpm_data(scenes.random_scene_3d(8000, "fluid", 1 / 64, seed=s)) for s in (1, 2)]
+    pipe = MpmPipeline()
+
+    def seconds(ds):
+        best = 1e9
+        for _ in range(7):
+            t0 = time.perf_counter()
+            for d in ds:
+                pipe.launch_step(d, 128)
+            for d in ds:
+                d.sync()
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    seconds(data)
+    one, two = seconds(data[:1]), seconds(data)
+    print(f"128 substeps of one scene {one * 1e6:.0f} us, of two {two * 1e6:.0f} us")
+    assert two <= 1.6 * one
+    for d in data:
+        d.close()
+
+
 @pytest.mark.parametrize("reported_by", ["sync", "positions", "timestep_bound"])
 def test_barrier_wait_is_bounded(cuda_lib, monkeypatch, reported_by):
     """The grid barrier made to wait for a CTA that never comes: the launch
