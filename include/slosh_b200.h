@@ -339,7 +339,8 @@ int slosh_sync(slosh_ctx *ctx, void *stream);
  * substep that keeps the previous grid launches 7 fewer: the reuse's
  * permutation update and touched-cell gather instead of the 9 build
  * kernels (slosh_get_stats counts both kinds of substep).  1: the scene's
- * substeps share launches of up to 32. */
+ * substeps share launches of up to 32 (not while a stage hook is set: those
+ * substeps run kernel by kernel). */
 uint32_t slosh_kernels_per_substep(const slosh_ctx *ctx);
 
 /* Runs `n_substeps` substeps with direct launches (not the CUDA graph) and a

@@ -1486,7 +1486,7 @@ int slosh_sync(slosh_ctx *c, void *stream) {
 
 uint32_t slosh_kernels_per_substep(const slosh_ctx *c) {
     if (!c) return 0;
-    if (takes_scene_steps(c)) return 1u;  // one launch covers up to STEPS_PER_LAUNCH substeps
+    if (!c->n_hooks && takes_scene_steps(c)) return 1u;  // one launch covers up to STEPS_PER_LAUNCH substeps
     // the full build's 9 kernels, P2G, the grid update, G2P and the rigid
     // update; with grid reuse the decision, and without conditional graphs
     // also the two reuse kernels, which return at once in a full build

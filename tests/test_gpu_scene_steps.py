@@ -19,6 +19,7 @@ from slosh_b200 import _lib, scenes
 from slosh_b200.pipeline import (
     MpmData,
     MpmPipeline,
+    MpmPipelineHooks,
     ParticleModel,
     RigidBody,
     SimulationParams,
@@ -161,6 +162,22 @@ def test_one_launch_matches_separate_kernels(cuda_lib, monkeypatch, name):
     assert ab.tobytes() == bb.tobytes()
     for k in ("n_blocks", "n_primary_blocks", "n_svd_fp64"):
         assert ast[k] == bst[k], k
+
+
+def test_kernels_counted_with_a_hook_set(cuda_lib):
+    """Substeps with a stage hook run kernel by kernel, and are counted so."""
+    counted = []
+
+    class Hooks(MpmPipelineHooks):
+        def after_p2g(self, data, stream, state):
+            counted.append(data.kernels_per_substep)
+
+    sc = _scene("fluid_odd")
+    data = scenes.build_mpm_data(sc)
+    MpmPipeline().launch_step(data, 1, hooks=Hooks())
+    data.sync()
+    assert data.kernels_per_substep == 1 and counted == [13]
+    data.close()
 
 
 def test_spread_scene_is_linear_in_its_blocks(cuda_lib, monkeypatch):
