@@ -180,9 +180,6 @@ template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile(
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t n) {
     asm volatile("barrier.sync %0, %1;\n" ::"r"(id), "r"(n) : "memory");
 }
-__device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t n) {
-    asm volatile("barrier.arrive %0, %1;\n" ::"r"(id), "r"(n) : "memory");
-}
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;

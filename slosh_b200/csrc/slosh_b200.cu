@@ -9,11 +9,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <string>
-#include <type_traits>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -51,8 +49,8 @@ struct slosh_ctx {
 
     // grid
     uint32_t *hkeys[2] = {nullptr, nullptr}, *hvals[2] = {nullptr, nullptr};
-    uint32_t *slot_counts = nullptr, *slot_total = nullptr, *blist_key = nullptr, *blist_slot = nullptr, *blist2_key = nullptr,
-             *blist2_slot = nullptr, *hist = nullptr, *hist_start = nullptr, *hist_coarse = nullptr, *tmp_key = nullptr,
+    uint32_t *slot_counts = nullptr, *slot_total = nullptr, *blist_key = nullptr, *blist_slot = nullptr,
+             *blist2_key = nullptr, *blist2_slot = nullptr, *hist = nullptr, *hist_start = nullptr, *hist_coarse = nullptr, *tmp_key = nullptr,
              *tmp_slot = nullptr, *bkey = nullptr, *bslot = nullptr, *bfirst = nullptr, *bnp = nullptr,
              *bcell = nullptr, *bcur = nullptr, *bnbh = nullptr, *bnbh_rev = nullptr;
     uint2 *bord = nullptr, *items = nullptr;
@@ -1048,7 +1046,8 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
         (st = dalloc(c, &c->staging, N)) || (st = dalloc(c, &c->bfirst2, cap)) || (st = dalloc(c, &c->bnp2, cap)) ||
         (st = dalloc(c, &c->bcell2, (size_t)cap * CELLS)) || (st = dalloc(c, &c->cell_delta, (size_t)cap * CELLS)) ||
         (st = dalloc(c, &c->touch, cap)) || (st = dalloc(c, &c->cur_touch, cap)) ||
-        (st = dalloc(c, &c->slot_total, hcap)) || (st = dalloc(c, &c->items, N / 32 + cap + 1)) || (st = dalloc(c, &c->reuse_cta, 2 * (size_t)REUSE_MAX_CTAS)) ||
+        (st = dalloc(c, &c->slot_total, hcap)) || (st = dalloc(c, &c->items, N / 32 + cap + 1)) ||
+        (st = dalloc(c, &c->reuse_cta, 2 * (size_t)REUSE_MAX_CTAS)) ||
         (st = dalloc(c, &c->touched_cells, (size_t)cap * CELLS)) || (st = dalloc(c, &c->bsrc, cap)))
         return fail_create(st);
     cudaMemset(c->hkeys[0], 0xff, hcap * 4);

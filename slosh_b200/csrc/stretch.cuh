@@ -112,7 +112,7 @@ template <int D> struct Stretch {
             return acc;
         };
         const float e00 = e(0, 0), e11 = e(1, 1), e01 = e(0, 1);
-        float limit, dp;
+        float dp;
         if constexpr (D == 3) {
             const float e22 = e(2, 2), e02 = e(0, 2), e12 = e(1, 2);
             m = (e00 + e11 + e22) * (1.f / 3.f);
@@ -127,7 +127,6 @@ template <int D> struct Stretch {
             X.square();
             dp = X.q - X.p;  // det(I + X) - 1
             detm1 = m * fmaf(m, m + 3.f, 3.f);
-            limit = 0.125f;
         } else {
             m = 0.5f * (e00 + e11);
             const float r = __fdividef(1.f, 1.f + m);
@@ -136,11 +135,10 @@ template <int D> struct Stretch {
             X.square();
             dp = -X.p;
             detm1 = m * (m + 2.f);
-            limit = 0.125f;
         }
         detm1 = fmaf(detm1, dp, detm1 + dp);
         const bool isotropic = X.p <= 1.5e-10f && fabsf(m) > 2e-5f;
-        return X.p <= limit && m > -0.6f && m < 4.f && !isotropic;
+        return X.p <= 0.125f && m > -0.6f && m < 4.f && !isotropic;
     }
 };
 
