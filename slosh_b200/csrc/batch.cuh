@@ -441,7 +441,7 @@ int slosh_batch_create(const slosh_batch_config *cfg, slosh_batch **out) {
         (st = dalloc(c, &c->coll[1], (size_t)cap * 64)) || (st = dalloc(c, &c->coll_id[0], (size_t)cap * 64)) ||
         (st = dalloc(c, &c->coll_id[1], (size_t)cap * 64)) || (st = dalloc(c, &c->bodies, b->max_bodies)) ||
         (st = dalloc(c, &c->body_imp, (size_t)b->max_bodies * 6)) ||
-        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 2)) || (st = dalloc(c, &c->small, 4)) ||
+        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 3)) || (st = dalloc(c, &c->small, 4)) ||
         (st = dalloc(c, &b->scene_nblk, b->max_scenes)) || (st = dalloc(c, &b->scene_bbase, b->max_scenes)) ||
         (st = dalloc(c, &b->scene_fill, b->max_scenes)) || (st = dalloc(c, &b->scenes_dev, b->max_scenes)) ||
         (st = dalloc(c, &b->n_dev, 1)) || (st = dalloc(c, &b->g2p_lists, (size_t)G2P_CLASSES * cap)) ||
@@ -845,7 +845,7 @@ int slosh_batch_timestep_bound(slosh_batch *b, uint32_t slot, float *dt_out, voi
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     const DevScene s = make_batch_scene(b, c->parity);
-    uint32_t *out = c->small + 3;
+    uint32_t *out = c->err + 2;
     const slosh_batch::Slot &sl = b->slots[slot];
     uint32_t u = 0;
     for (;;) {
@@ -854,9 +854,8 @@ int slosh_batch_timestep_bound(slosh_batch *b, uint32_t slot, float *dt_out, voi
         if (c->dim == 3) k_timestep_bound<3, true><<<g, 256, 0, st>>>(s, slot, start, span, out);
         else k_timestep_bound<2, true><<<g, 256, 0, st>>>(s, slot, start, span, out);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&u, out, 4, cudaMemcpyDeviceToHost, st));
         uint32_t e = 0;
-        if (int r = wait_and_read_error(c, st, &e)) return r;
+        if (int r = wait_and_read_error(c, st, &e, &u)) return r;
         if (e == 0u || b->misplaced) break;
         // an error that is still to be reported: storage may have lost
         // particles, so the scene may lie elsewhere

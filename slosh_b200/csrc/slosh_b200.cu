@@ -106,7 +106,9 @@ struct slosh_ctx {
     uint32_t *mesh_idx = nullptr;
     uint32_t n_meshes = 0;
     Counters *ctr = nullptr;
-    uint32_t *err = nullptr;    // [0] error bits, [1] active blocks of the last one-launch substep
+    // [0] error bits, [1] active blocks of the last one-launch substep, [2] a
+    // time step bound: what a wait brings back in one copy
+    uint32_t *err = nullptr;
     uint32_t blocks_seen = 0;   // err[1] at the last wait (0: none since the upload)
     uint32_t *small = nullptr;  // [0] n_mat, [1] scene flags, [2] debug total
     uint32_t parity = 0;
@@ -874,14 +876,16 @@ int check_device_error(slosh_ctx *c) {
 
 // Waits for the stream's work and reads the error bits with the same wait:
 // the end of every download (a copy of its own after the wait was a second
-// round trip of about 10 us).  The word behind them says how many blocks the
-// scene has, for the next launches' CTAs.
-int wait_and_read_error(slosh_ctx *c, cudaStream_t st, uint32_t *e) {
-    uint32_t w[2] = {0, 0};
-    CK(cudaMemcpyAsync(w, c->err, 8, cudaMemcpyDeviceToHost, st));
+// round trip of about 10 us).  The words behind them come with the same copy:
+// how many blocks the scene has, for the next launches' CTAs, and the time step
+// bound for the calls that ask for it.
+int wait_and_read_error(slosh_ctx *c, cudaStream_t st, uint32_t *e, uint32_t *bound = nullptr) {
+    uint32_t w[3] = {0, 0, 0};
+    CK(cudaMemcpyAsync(w, c->err, bound ? 12 : 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     *e = w[0];
     c->blocks_seen = w[1];
+    if (bound) *bound = w[2];
     return SLOSH_OK;
 }
 int wait_and_check(slosh_ctx *c, cudaStream_t st) {
@@ -1042,7 +1046,7 @@ int slosh_ctx_create(const slosh_config *cfg, slosh_ctx **out) {
         (st = dalloc(c, &c->coll[1], (size_t)cap * 64)) || (st = dalloc(c, &c->coll_id[0], (size_t)cap * 64)) ||
         (st = dalloc(c, &c->coll_id[1], (size_t)cap * 64)) || (st = dalloc(c, &c->bodies, MAX_BODIES)) ||
         (st = dalloc(c, &c->body_imp, (size_t)MAX_BODIES * 6)) ||
-        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 2)) || (st = dalloc(c, &c->small, 4)) ||
+        (st = dalloc(c, &c->ctr, 1)) || (st = dalloc(c, &c->err, 3)) || (st = dalloc(c, &c->small, 4)) ||
         (st = dalloc(c, &c->staging, N)) || (st = dalloc(c, &c->bfirst2, cap)) || (st = dalloc(c, &c->bnp2, cap)) ||
         (st = dalloc(c, &c->bcell2, (size_t)cap * CELLS)) || (st = dalloc(c, &c->cell_delta, (size_t)cap * CELLS)) ||
         (st = dalloc(c, &c->touch, cap)) || (st = dalloc(c, &c->cur_touch, cap)) ||
@@ -1700,15 +1704,14 @@ int slosh_timestep_bound(slosh_ctx *c, float *dt_out, void *stream) {
     CK(cudaSetDevice(c->device));
     cudaStream_t st = pick(c, stream);
     const DevScene s = make_scene(c, c->parity, false);
-    uint32_t *slot = c->small + 3;
+    uint32_t *slot = c->err + 2;
     CK(cudaMemsetAsync(slot, 0xff, 4, st));
     const uint32_t g = grid_for(c->n, 256, (uint32_t)c->sm_count * 16);
     if (c->dim == 3) k_timestep_bound<3><<<g, 256, 0, st>>>(s, 0u, 0u, c->n, slot);
     else k_timestep_bound<2><<<g, 256, 0, st>>>(s, 0u, 0u, c->n, slot);
     CK(cudaGetLastError());
     uint32_t u = 0, e = 0;
-    CK(cudaMemcpyAsync(&u, slot, 4, cudaMemcpyDeviceToHost, st));
-    if (int r = wait_and_read_error(c, st, &e)) return r;
+    if (int r = wait_and_read_error(c, st, &e, &u)) return r;
     if (e & ERR_BARRIER) return report_device_error(c, e);  // the bound is of no known state
     *dt_out = (float)u / TIMESTEP_FLOAT_TO_INT;  // GpuTimestepBounds::computed_dt
     return SLOSH_OK;
