@@ -249,8 +249,11 @@ __device__ __forceinline__ void model_update(const Material &mat, uint32_t tag, 
         // are made of it, so another arithmetic gives visibly other stresses
         // there (matrix polynomials as in stretch.cuh: C up to 9 % apart in
         // the first substeps of a column, if closer to 64 bits; G2P of the
-        // 4.74 M-particle column 247 us instead of 307).  Without a plastic
-        // model (its lambda is 0) sand is purely elastic.
+        // 4.74 M-particle column 247 us instead of 307).  Rounding in other
+        // stages reaches it too: the order of P2G's sums moves the C of a
+        // two-way column by 7e-4 of its norm, at the same distance from 64
+        // bits.  Without a plastic model (its lambda is 0) sand is purely
+        // elastic.
         const bool plastic = mat.p[7] != 0.f;
         if (tag == SLOSH_MODEL_SAND_LINEAR || plastic) {
             SvdD<D> sv;

@@ -561,8 +561,9 @@ constexpr uint32_t STEPS_PER_LAUNCH = 32;
 // 3,375 sand particles 38.8 and 38.5 (32 CTAs), 8,000 39.1 and 38.7 (50), 10,648
 // 40.0 and 40.6 (64), 15,625 40.3 and 40.8 (94); larger scenes need the SMs
 // (59,319 fluid particles 43 on 148, 52 on 111, 55 on 74).  Two and four scenes
-// of 8,000 fluid particles on as many streams: 73 and 146 where each takes every
-// SM, 38 and 75 on 74 CTAs, 70 and 99 as separate kernels.
+// on as many streams, microseconds a substep of all: of 8,000 fluid particles
+// 74 and 147 where each takes every SM, 38 and 76 so, 69 and 99 as separate
+// kernels; of 29,791 80 and 160 both ways, 81 and 118 as separate kernels.
 constexpr uint32_t STEPS_PARTICLES_PER_CTA = 168, STEPS_BLOCKS_PER_CTA = 2, STEPS_MIN_CTAS = 32;
 uint32_t steps_grid(const slosh_ctx *c) {
     const uint32_t all = (uint32_t)c->sm_count;
