@@ -259,3 +259,17 @@ def test_bench_launch_accounting():
     st1 = {"n_grid_reuses": 0, "n_grid_rebuilds": 0, "conditional_graphs": 0}
     launches, _ = bench.timed_launches(SimpleNamespace(kernels_per_substep=13), st1, st1, 1000)
     assert launches == 13000
+
+
+def test_division_by_three_from_the_reciprocal():
+    """The Drucker-Prager kernel divides by 3 with a multiplication by the
+    rounded reciprocal and one correction by the remainder (models.cuh): the
+    correctly rounded quotient, for every mantissa.  In double precision the
+    remainder and the corrected quotient are exact before their one rounding."""
+    third = np.float32(1.0) / np.float32(3.0)
+    for exponent in (0, 1):  # the quotient's mantissa depends on the operand's alone
+        x = ((np.arange(1 << 23, 1 << 24, dtype=np.uint32)).astype(np.float32)) * np.float32(2.0**exponent)
+        q = x * third
+        r = (x.astype(np.float64) - 3.0 * q.astype(np.float64)).astype(np.float32)
+        got = (q.astype(np.float64) + r.astype(np.float64) * np.float64(third)).astype(np.float32)
+        assert np.array_equal(got, x / np.float32(3.0))
