@@ -144,9 +144,11 @@ template <int D>
 __device__ __forceinline__ void drucker_prager(float *st, const float *p, SvdD<D> &sv, float (&F)[D][D]) {
     const float ha = p[0], hb = p[1], hc = p[2], hd = p[3], lambda = p[4], mu = p[5];
     const float q = st[1];
-    // The friction angle and the cone slope only place the yield surface:
-    // the hardware approximations (a few ulp) are used for them; the terms
-    // that enter F and the plastic state keep the correctly rounded forms.
+    // The friction angle and the cone slope only place the yield surface, and
+    // gamma with the share of the deviator it takes away measures the distance
+    // to it: the hardware approximations (a few ulp) are used for them.  The
+    // strains, exponentials and the plastic state have logf, expf, sqrtf and
+    // correctly rounded quotients.
     const float angle = ha + (hb * q - hd) * __expf(-hc * q);
     const float s_angle = __sinf(angle);
     const float alpha = __fdividef(sqrtf(2.0f / 3.0f) * (2.0f * s_angle), 3.0f - s_angle);
